@@ -55,8 +55,8 @@ FRAGMENT_BYTES = 8           # one 64-bit depth-test reduction per fragment
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "dram_bytes_c2_frame.txt")
 # (k_raster_alpha<K> launches only for scenes with alpha-clip meshes)
 STAGE_KERNELS = {
-    "raster": ("k_raster<0, 3>", "k_raster_alpha<0>", "k_raster_big<0>", "k_hiz", "k_occlusion_filter"),
-    "shadow_raster": ("k_raster<1, 3>", "k_raster_alpha<1>", "k_raster_big<1>"),
+    "raster": ("k_raster<0>", "k_raster_alpha<0>", "k_raster_big<0>", "k_hiz", "k_occlusion_filter"),
+    "shadow_raster": ("k_raster<1>", "k_raster_alpha<1>", "k_raster_big<1>"),
     "resolve": ("k_resolve<1>",),
     "cull_meshlets": ("k_cull_meshlets",),
     "depth_fit": ("k_depth_reduce_fit",),

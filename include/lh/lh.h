@@ -246,8 +246,8 @@ typedef struct lh_tuning {
                                  chunk_cols pixels, one warp each) */
     float cull_blocks_per_sm; /* meshlet-cull blocks per SM (per-stage schedule); blocks per SM (persistent) */
     uint32_t schedule;        /* LH_SCHEDULE_* */
-    uint32_t raster_batch;    /* meshlets a raster warp claims per atomic (0: 4 when the views hold more than
-                                 256 meshlets per warp of the grid, else 1) */
+    uint32_t raster_batch;    /* meshlets a raster warp claims per atomic, at most 8 (0: from 8 down to 1 as the
+                                 meshlets of the views run out) */
     uint32_t occlusion_px;    /* two-pass occlusion raster of the visibility views: opaque meshlets whose
                                  bounding sphere projects to a radius above this many pixels are drawn
                                  first, the hierarchical depth of what they wrote is built, and every other

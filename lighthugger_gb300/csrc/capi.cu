@@ -51,7 +51,7 @@ struct lh_ctx {
     uint8_t* d_sectors = nullptr;
     MeshletReference* d_refs = nullptr;
     RasterDraw* d_rdraws = nullptr;  // the raster's per-slot draw records
-    uint32_t* d_lists = nullptr;     // occlusion lists of the visibility views (3 * max_draws words each)
+    uint32_t* d_lists = nullptr;     // the views' raster lists (4 * max_draws words each)
     uint32_t* d_hiz = nullptr;       // hierarchical depth of the visibility views (pool)
     size_t hiz_words = 0;
     uint8_t* d_draws = nullptr;
@@ -245,10 +245,10 @@ void build_views(lh_ctx* c, uint32_t n_probes, const Uniforms* probe_uniforms) {
         vw.inst_status = reinterpret_cast<uint64_t*>(r + 4 * kClaimWords);
         vw.ml_status = reinterpret_cast<uint64_t*>(r + 4 * kClaimWords + 8 * (size_t)n_inst_tiles);
         vw.ml_tile_cap = ml_tiles;
+        vw.lists = c->d_lists + (size_t)v * 4 * cfg.max_draws;
         if (!cascade) {
-            // occlusion lists, and the view's hierarchical depth from the
-            // pool while it lasts (a view without one culls nothing)
-            vw.lists = c->d_lists + (size_t)v * 3 * cfg.max_draws;
+            // the view's hierarchical depth from the pool while it lasts (a
+            // view without one culls nothing)
             vw.hiz_rx = (vw.width + kHizRegion - 1) / kHizRegion;
             vw.hiz_ry = (vw.height + kHizRegion - 1) / kHizRegion;
             const size_t words = (size_t)vw.hiz_rx * vw.hiz_ry * 65;
@@ -299,6 +299,7 @@ FrameDev frame_dev(const lh_ctx* c, uint32_t n_views, uint32_t n_instances) {
         f.chunk_shift[k][1] = (uint32_t)__builtin_ctz(c->tuning.chunk_cols[k]);
     }
     f.backward_rows = c->tuning.backward_rows;
+    f.neg_zero2 = 0x8000000080000000ull;
     return f;
 }
 
@@ -535,7 +536,7 @@ lh_status lh_create(const lh_config* config, lh_ctx** out) {
     if (e == cudaSuccess) e = dalloc(c, &c->d_sectors, c->sector_bytes * c->max_views);
     if (e == cudaSuccess) e = dalloc(c, &c->d_refs, sizeof(MeshletReference) * 2 * (size_t)cfg.max_draws * c->max_views);
     if (e == cudaSuccess) e = dalloc(c, &c->d_rdraws, sizeof(RasterDraw) * 2 * (size_t)cfg.max_draws * c->max_views);
-    if (e == cudaSuccess) e = dalloc(c, &c->d_lists, sizeof(uint32_t) * 3 * (size_t)cfg.max_draws * (1 + cfg.max_probes));
+    if (e == cudaSuccess) e = dalloc(c, &c->d_lists, sizeof(uint32_t) * 4 * (size_t)cfg.max_draws * c->max_views);
     // hierarchical depth: the main view, and the probes' total pixels in 64 x
     // 64 regions with room for each probe's partial regions
     c->hiz_words = align_up(((W + kHizRegion - 1) / kHizRegion) * ((H + kHizRegion - 1) / kHizRegion) * 65, 64) +
@@ -907,7 +908,7 @@ lh_status lh_read_status(lh_ctx* c, lh_device_status* out) {
         e = cudaMemcpy(claim, c->h_views[0].claim, sizeof(claim), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(c, e, "status read");
         out->occlusion[0] = claim[kClaimOccluders];
-        out->occlusion[1] = claim[kClaimSurvivorsOpaque];
+        out->occlusion[1] = claim[kClaimSurvivorsOpaque] + claim[kClaimGeneral];
         out->occlusion[2] = claim[kClaimSurvivorsAlpha];
     }
     out->n_views = c->n_views_last;

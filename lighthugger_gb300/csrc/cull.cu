@@ -39,7 +39,8 @@ __global__ void __launch_bounds__(kMlThreads, LH_ML_MIN_BLOCKS)
     pdl_enter();
     if (blockIdx.x == 0 && threadIdx.x < kStWords) {
         const uint32_t w = threadIdx.x;
-        if (w >= kStClipCount && w <= kStRasterClaimAlpha && w != kStMlClaim && w != kStBarrier) f.status[w] = 0u;
+        if ((w >= kStClipCount && w <= kStRasterClaimAlpha && w != kStMlClaim && w != kStBarrier) || w == kStWholeClaim)
+            f.status[w] = 0u;
     }
     phase_cull_meshlets(f, view_begin, n_views, &f.status[kStMlClaim]);
 }

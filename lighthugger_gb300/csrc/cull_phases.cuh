@@ -107,6 +107,14 @@ __device__ __forceinline__ float bounding_radius(const float4 (&c)[4], float r) 
     return r * sqrtf(lam) * (1.0f + 1.0f / 65536.0f);
 }
 
+// atomicAdd(counter, 1) by each of the warp's active lanes, as one atomic.
+__device__ __forceinline__ uint32_t count_up(uint32_t* counter) {
+    const uint32_t m = __activemask(), lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    uint32_t first = 0;
+    if (lane == leader) first = atomicAdd(counter, __popc(m));
+    return __shfl_sync(m, first, leader) + __popc(m & ((1u << lane) - 1u));
+}
+
 // The raster's record of a visible meshlet (the scene records it reads were
 // loaded moments earlier by the same thread, so these loads mostly hit):
 // the addresses of its vertex data, its world-space bounding sphere, and --
@@ -131,6 +139,8 @@ __device__ __forceinline__ RasterDraw raster_draw_of(const FrameDev& f, const Vi
     r.instance = ref.instance_index;
     // counts = triangle_count | index_count << 8
     r.bits = ((counts >> 8) & 0xFFu) | ((counts & 0xFFu) << 8) | (mflags << 16);
+    const uint32_t nv = (counts >> 8) & 0xFFu, nt = counts & 0xFFu;
+    if (nv == 0 || nv > MAX_MESHLET_UNIQUE_VERTICES || nt > MAX_MESHLET_TRIANGLES || (r.micro & 3)) r.bits |= kDrawGeneral;
     // world sphere: transform * centre, radius through the linear part
     float4 tc[4];
     const float4* tsrc = reinterpret_cast<const float4*>(inst);
@@ -151,19 +161,28 @@ __device__ __forceinline__ RasterDraw raster_draw_of(const FrameDev& f, const Vi
     // small views (probes): a meshlet whose sphere reaches no pixel centre
     // is common there, and the raster skips it before its vertices (in
     // large views the test would cost the cull more than it saves)
+    const bool occlusion = f.occlusion_px && vw->kind == kViewVisibility;
     if (vw->width * vw->height <= kNoCentreTestPixels && sphere_misses_centres(vp, wx, wy, wz, R, vw->width, vw->height)) {
         r.bits |= kDrawNoCentre;
-        return r;
-    }
-    if (f.occlusion_px && !alpha && vw->kind == kViewVisibility && vw->lists) {
+    } else if (vw->kind == kViewVisibility) {
         const lh_mat4& pv = u.combined_perspective_view;
         const float w = ((pv.cols[0].w * wx + pv.cols[1].w * wy) + pv.cols[2].w * wz) + pv.cols[3].w;
-        const float focal_px = fabsf(u.perspective.cols[1].y) * 0.5f * (float)vw->height;
-        if (!(w > R) || R * focal_px > (float)f.occlusion_px * (w - R)) {
+        const float radius_px = R * (fabsf(u.perspective.cols[1].y) * 0.5f * (float)vw->height);  // times 1 / (w - R)
+        if (!(w > R) || radius_px > kSmallRadiusPx * (w - R)) r.bits |= kDrawGeneral;
+        if (occlusion && !alpha && (!(w > R) || radius_px > (float)f.occlusion_px * (w - R))) {
             r.bits |= kDrawOccluder;
-            const uint32_t pos = atomicAdd(&vw->claim[kClaimOccluders], 1u);
+            const uint32_t pos = count_up(&vw->claim[kClaimOccluders]);
             if (pos < f.max_draws) vw->lists[pos] = slot;
         }
+    } else {
+        // an orthographic cascade: the matrix's y row scales to ndc
+        const float sx = vp.cols[0].y, sy = vp.cols[1].y, sz = vp.cols[2].y;
+        if (!(R * sqrtf(sx * sx + sy * sy + sz * sz) * 0.5f * (float)vw->height <= kSmallRadiusPx)) r.bits |= kDrawGeneral;
+    }
+    // (the occlusion raster lists its general meshlets after the depth test)
+    if ((r.bits & kDrawGeneral) && !alpha && !occlusion) {
+        const uint32_t pos = count_up(&vw->claim[kClaimGeneral]);
+        if (pos < f.max_draws) vw->lists[(size_t)3 * f.max_draws + pos] = slot;
     }
     return r;
 }

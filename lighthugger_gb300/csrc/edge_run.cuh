@@ -62,40 +62,51 @@ LH_ER_HD int32_t f32_floor_to_i32(float x) {
 // in 1/256 pixels), shared by every row of the triangle's chunks (0 for dy = 0).
 LH_ER_HD float run_inv_step(int32_t dy) { return dy == 0 ? 0.0f : approx_rcp(std::fabs((float)dy) * 256.0f); }
 
+// The magnitude of a 32-bit value as float, for the 32-bit estimate.
+LH_ER_HD float abs_to_f32(int32_t v) { return (float)(uint32_t)(v < 0 ? 0u - (uint32_t)v : (uint32_t)v); }
+
 // Narrow [lo, hi] (pixels 0 .. n-1 of the row, n <= 256) to the pixels where
 // e0 + k * dx >= bias; an empty result has lo > hi.  inv = run_inv_step(dy).
-LH_ER_HD void clip_run(int64_t e0, int64_t dx, int64_t bias, int32_t n, float inv, int32_t& lo, int32_t& hi) {
+// I = int32_t: for triangles whose edge products inside the box fit 32 bits
+// (ext_x * ext_y < 2^30, the row inside the box: |e0|, |e0 + k dx| < 2^31 and
+// (n - 1) |dx| < 2^30), half the instructions of the 64-bit form.
+template <class I>
+LH_ER_HD void clip_run_as(I e0, I dx, I bias, int32_t n, float inv, int32_t& lo, int32_t& hi) {
     if (dx == 0) {
         if (e0 < bias) hi = -1;
         return;
     }
     if (dx > 0) {
         // first passing pixel: ceil((bias - e0) / dx)
-        const int64_t need = bias - e0;
+        const I need = bias - e0;
         if (need <= 0) return;
-        if (need > (int64_t)(n - 1) * dx) {
+        if (need > (I)(n - 1) * dx) {
             hi = -1;
             return;
         }
         int32_t k = f32_ceil_to_i32(abs_to_f32(need) * inv);
         k = k < 1 ? 1 : (k > n - 1 ? n - 1 : k);
-        if (e0 + (int64_t)(k - 1) * dx >= bias) k--;
-        else if (e0 + (int64_t)k * dx < bias) k++;
+        if (e0 + (I)(k - 1) * dx >= bias) k--;
+        else if (e0 + (I)k * dx < bias) k++;
         if (k > lo) lo = k;
     } else {
         // last passing pixel: floor((e0 - bias) / -dx)
-        const int64_t room = e0 - bias;
+        const I room = e0 - bias;
         if (room < 0) {
             hi = -1;
             return;
         }
-        if (room >= (int64_t)(n - 1) * -dx) return;
+        if (room >= (I)(n - 1) * -dx) return;
         int32_t k = f32_floor_to_i32(abs_to_f32(room) * inv);
         k = k < 0 ? 0 : (k > n - 2 ? n - 2 : k);
-        if (e0 + (int64_t)(k + 1) * dx >= bias) k++;
-        else if (e0 + (int64_t)k * dx < bias) k--;
+        if (e0 + (I)(k + 1) * dx >= bias) k++;
+        else if (e0 + (I)k * dx < bias) k--;
         if (k < hi) hi = k;
     }
+}
+
+LH_ER_HD void clip_run(int64_t e0, int64_t dx, int64_t bias, int32_t n, float inv, int32_t& lo, int32_t& hi) {
+    clip_run_as<int64_t>(e0, dx, bias, n, inv, lo, hi);
 }
 
 }  // namespace lh

@@ -282,6 +282,7 @@ struct TriSetup {
     uint32_t verts;  // alpha-tested: meshlet vertices m0 | m1 << 8 | m2 << 16
 };
 constexpr uint32_t kBiasAlpha = 16u;
+constexpr uint32_t kBiasWhole = 32u;  // BigTri: taken whole by one warp, not by chunks
 
 __device__ __forceinline__ bool top_left(int32_t ax, int32_t ay, int32_t bx, int32_t by) {
     int32_t dy = by - ay, dx = bx - ax;
@@ -429,9 +430,7 @@ __device__ __forceinline__ bool cover(const TriSetup& t, int32_t px, int32_t py,
 // bits in a u32 shadow target (LESS).  The atomics return nothing (RED), so
 // a warp never waits on the L2 round trip of a fragment.
 template <int KIND>
-__device__ __forceinline__ void write_fragment(void* target, uint32_t W, int32_t px, int32_t py, float depth,
-                                               uint32_t id) {
-    size_t pix = (size_t)py * W + px;
+__device__ __forceinline__ void write_pixel(void* target, size_t pix, float depth, uint32_t id) {
     if (KIND == 0) {
         const unsigned long long key = ((unsigned long long)f2u(depth) << 32) | id;
         asm volatile("red.relaxed.gpu.global.max.u64 [%0], %1;" ::"l"(reinterpret_cast<unsigned long long*>(target) + pix),
@@ -440,6 +439,11 @@ __device__ __forceinline__ void write_fragment(void* target, uint32_t W, int32_t
         asm volatile("red.relaxed.gpu.global.min.u32 [%0], %1;" ::"l"(reinterpret_cast<uint32_t*>(target) + pix),
                      "r"(f2u(depth)));
     }
+}
+template <int KIND>
+__device__ __forceinline__ void write_fragment(void* target, uint32_t W, int32_t px, int32_t py, float depth,
+                                               uint32_t id) {
+    write_pixel<KIND>(target, (size_t)py * W + px, depth, id);
 }
 
 // One pixel of the HDR target: RGBA32F, or RGBA16F (round to nearest even,

@@ -40,7 +40,7 @@ struct __align__(16) RasterDraw {
     uint64_t indices;    // MeshInfo.indices + Meshlet.index_offset elements
     uint64_t micro;      // MeshInfo.micro_indices + Meshlet.triangle_offset
     uint32_t instance;   // MeshletReference.instance_index
-    uint32_t bits;       // index_count | triangle_count << 8 | MeshInfo.flags << 16 | kDrawNoCentre | kDrawOccluder
+    uint32_t bits;       // index_count | triangle_count << 8 | MeshInfo.flags << 16 | kDrawGeneral | kDrawNoCentre | kDrawOccluder
     float sphere[4];     // world-space sphere holding every vertex of the meshlet (centre, radius)
 };
 static_assert(sizeof(RasterDraw) == 48, "RasterDraw layout");
@@ -48,12 +48,24 @@ static_assert(sizeof(RasterDraw) == 48, "RasterDraw layout");
 // visibility view with occlusion culling, opaque, large on screen).
 constexpr uint32_t kDrawOccluder = 1u << 31;
 constexpr uint32_t kDrawNoCentre = 1u << 30;  // the world sphere reaches no pixel centre of the view
+// Not for the raster's small path (raster_meshlet_small): the world sphere
+// projects to a radius above kSmallRadiusPx pixels or reaches the camera
+// plane (a hint: its vertices most likely span more than that path's 127
+// pixels, and finding out costs their transform), the meshlet is empty or
+// malformed, or its micro indices are not 4-byte aligned.
+constexpr uint32_t kDrawGeneral = 1u << 29;
+#ifndef LH_SMALL_RADIUS_PX
+#define LH_SMALL_RADIUS_PX 80.0f
+#endif
+constexpr float kSmallRadiusPx = LH_SMALL_RADIUS_PX;
 constexpr uint32_t kNoCentreTestPixels = 512u * 512u;  // views up to this size test it (sphere_box.cuh)
 
 // Per-view lists of the two-pass occlusion raster of visibility views
-// (ViewDev::lists, 3 * max_draws words): draw slots of the occluders, then
+// (ViewDev::lists, 4 * max_draws words): draw slots of the occluders, then
 // of the opaque and the alpha-clip meshlets that survive the hierarchical
-// depth test.  Their counts are ViewDev::claim[kClaimOccluders ...].
+// depth test, then of the opaque kDrawGeneral ones (survivors; in a view
+// without the occlusion raster, all of them).  Their counts are
+// ViewDev::claim[kClaimOccluders ...].
 enum RasterList : uint32_t { kListAll = 0, kListOccluders = 1, kListSurvivors = 2 };
 enum ClaimWord : uint32_t {
     kClaimInstTiles = 0,
@@ -61,6 +73,7 @@ enum ClaimWord : uint32_t {
     kClaimOccluders = 2,       // entries of the occluder list
     kClaimSurvivorsOpaque = 3,
     kClaimSurvivorsAlpha = 4,
+    kClaimGeneral = 5,
     kClaimWords = 8
 };
 // Hierarchical depth of a visibility view (ViewDev::hiz): level 0 holds the
@@ -86,7 +99,7 @@ struct ViewDev {
     uint32_t* claim;            // per-frame zeroed kClaimWords: tile claims, occlusion list counts
     uint32_t section_base;      // firstInstance offset of this view's reference section
     uint32_t ml_tile_cap;       // capacity of ml_status
-    uint32_t* lists;            // visibility views: occluder / survivor draw-slot lists (3 * max_draws)
+    uint32_t* lists;            // draw-slot lists of the raster passes (RasterList; 4 * max_draws)
     uint32_t* hiz;              // visibility views with occlusion culling: hierarchical depth, else null
     uint32_t hiz_rx, hiz_ry;    // 64 x 64-pixel regions of the view
 };
@@ -114,13 +127,14 @@ enum StatusWord : uint32_t {
     kStRasterClaim = 2,
     kStBigClaim = 3,
     kStReduceDone = 4,
-    // word 5 is unused
+    kStRasterClaimGeneral = 5,  // raster claims of the general loop
     kStMlClaim = 6,    // meshlet-cull (view, tile) claims
     kStBarrier = 7,    // grid barrier of the persistent kernel
     kStBigPacked = 8,  // u64 (words 8-9): big-triangle count << 40 | chunk count
     kStRasterClaimAlpha = 10,  // raster claims of the alpha-clip class
     kStFragVis = 11,     // fragments written this frame, visibility views (statistics)
     kStFragShadow = 12,  // the same, shadow views
+    kStWholeClaim = 13,  // chunk kernel: claims of the triangles taken whole
     kStWords = 16
 };
 
@@ -150,6 +164,7 @@ struct FrameDev {
     uint32_t occlusion_px;      // occluder threshold (projected sphere radius, pixels); 0: no occlusion culling
     uint32_t chunk_shift[2][2]; // [pass: visibility, shadow][log2 rows, log2 columns] of a big-triangle chunk
     uint32_t backward_rows;     // pixel rows of a resolve-adjoint tile: 4, 8 or 16
+    uint64_t neg_zero2;         // two -0.0f, as a value the compiler cannot see (packed multiplies, raster_phases.cuh)
     uint32_t scene_alpha;       // some mesh of the scene is alpha clip (else no alpha-class launch)
 };
 

@@ -45,13 +45,18 @@ __device__ bool grid_barrier(const FrameDev& f, uint32_t& epoch) {
 __device__ void reset_raster_words(const FrameDev& f) {
     for (uint32_t w = kStClipCount + threadIdx.x; w <= kStRasterClaimAlpha; w += blockDim.x)
         if (w != kStBarrier && w != kStReduceDone) f.status[w] = 0u;
+    if (threadIdx.x == 0) f.status[kStWholeClaim] = 0u;
 }
 
 constexpr int kPersistentThreads = 256;
 
-__global__ void __launch_bounds__(kPersistentThreads, 3) k_frame_persistent(FrameDev f, uint32_t n_persp,
+__global__ void __launch_bounds__(kPersistentThreads, 3) k_frame_persistent(const __grid_constant__ FrameDev f, uint32_t n_persp,
                                                                            RasterTune tune) {
-    __shared__ RasterSmemAlpha s_raster;  // reused by every raster phase
+    __shared__ union {
+        RasterSmemSmall small;
+        RasterSmemAlpha alpha;
+        BigSmem big;
+    } s_raster;  // reused by every raster phase
     uint32_t epoch = 0;
     const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, gstride = (uint64_t)gridDim.x * blockDim.x;
     const uint32_t n_views = n_persp + 4;
@@ -68,23 +73,22 @@ __global__ void __launch_bounds__(kPersistentThreads, 3) k_frame_persistent(Fram
     if (f.occlusion_px) {
         // occluders and their chunks, hierarchical depth, the depth test of
         // the other meshlets, then the survivors
-        phase_raster<0, false>(f, 0, n_persp, tune, &f.status[kStRasterClaim], s_raster, nullptr, kListOccluders);
+        phase_raster_general<0, false>(f, 0, n_persp, tune, s_raster.small, nullptr, kListOccluders);
         if (!grid_barrier(f, epoch)) return;
-        phase_raster_big<0>(f);
+        phase_raster_big<0>(f, s_raster.big);
         if (!grid_barrier(f, epoch)) return;
         phase_hiz(f, 0, n_persp);
         if (!grid_barrier(f, epoch)) return;
         phase_occlusion_filter(f, 0, n_persp, gtid, gstride);
         if (!grid_barrier(f, epoch)) return;
-        phase_raster<0, false>(f, 0, n_persp, tune, &f.status[kStRasterClaim], s_raster, nullptr, kListSurvivors);
-        phase_raster<0, true>(f, 0, n_persp, tune, &f.status[kStRasterClaimAlpha], s_raster, s_raster.av,
-                              kListSurvivors);
+        phase_raster<0>(f, 0, n_persp, tune, s_raster.small, kListSurvivors);
+        phase_raster_general<0, true>(f, 0, n_persp, tune, s_raster.alpha, s_raster.alpha.av, kListSurvivors);
     } else {
-        phase_raster<0, false>(f, 0, n_persp, tune, &f.status[kStRasterClaim], s_raster, nullptr);
-        phase_raster<0, true>(f, 0, n_persp, tune, &f.status[kStRasterClaimAlpha], s_raster, s_raster.av);
+        phase_raster<0>(f, 0, n_persp, tune, s_raster.small, kListAll);
+        phase_raster_general<0, true>(f, 0, n_persp, tune, s_raster.alpha, s_raster.alpha.av, kListAll);
     }
     if (!grid_barrier(f, epoch)) return;
-    phase_raster_big<0>(f);
+    phase_raster_big<0>(f, s_raster.big);
     if (!grid_barrier(f, epoch)) return;
     // depth range of the main view, then the cascade fit
     phase_depth_reduce(f, gtid, gstride);
@@ -100,10 +104,10 @@ __global__ void __launch_bounds__(kPersistentThreads, 3) k_frame_persistent(Fram
     if (!grid_barrier(f, epoch)) return;
     phase_cull_meshlets(f, n_persp, 4, &f.status[kStMlClaim]);
     if (!grid_barrier(f, epoch)) return;
-    phase_raster<1, false>(f, n_persp, 4, tune, &f.status[kStRasterClaim], s_raster, nullptr);
-    phase_raster<1, true>(f, n_persp, 4, tune, &f.status[kStRasterClaimAlpha], s_raster, s_raster.av);
+    phase_raster<1>(f, n_persp, 4, tune, s_raster.small, kListAll);
+    phase_raster_general<1, true>(f, n_persp, 4, tune, s_raster.alpha, s_raster.alpha.av, kListAll);
     if (!grid_barrier(f, epoch)) return;
-    phase_raster_big<1>(f);
+    phase_raster_big<1>(f, s_raster.big);
 }
 
 int g_persistent_blocks_per_sm = -1;

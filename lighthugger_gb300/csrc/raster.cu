@@ -3,10 +3,7 @@
 #include "raster_phases.cuh"
 
 #ifndef LH_RASTER_MIN_BLOCKS
-#define LH_RASTER_MIN_BLOCKS 3  // resident blocks of k_raster per SM (registers: 65536 / 256 / this)
-#endif
-#ifndef LH_RASTER_MULTIVIEW_MIN_BLOCKS
-#define LH_RASTER_MULTIVIEW_MIN_BLOCKS 4  // the same when one launch rasterises several visibility views
+#define LH_RASTER_MIN_BLOCKS 4  // resident blocks of k_raster per SM (registers: 65536 / 256 / this)
 #endif
 #ifndef LH_RASTER_BIG_MIN_BLOCKS
 #define LH_RASTER_BIG_MIN_BLOCKS 4  // the same for the chunk kernel k_raster_big
@@ -15,33 +12,39 @@
 namespace lh {
 namespace {
 
-// MINB resident blocks per SM.  One large view (the main visibility view,
-// the cascades) runs best at 3 (80 registers, no spills); a launch over many
-// small views (main + probes: mostly meshlets whose vertices span no pixel
-// centre, bound by the latency of their loads) at 4 (64 registers): 3.66 ->
-// 3.53 ms for main + 32 probes + 4 cascades, while 4 costs the lone main
-// view 0.328 -> 0.343 ms.
-template <int KIND, int MINB>
-__global__ void __launch_bounds__(kRasterWarps * 32, MINB) k_raster(FrameDev f, uint32_t view_begin, uint32_t n_views,
-                                                                   RasterTune tune, uint32_t list) {
+// The opaque class.  Four resident blocks per SM (64 registers): the 1080p
+// frame 0.616 ms at three, 0.606 at four, 0.624 at five; the 4K stress frame
+// 18.3 / 17.8 / 18.0; main + 32 probes 2.28 / 2.29 / 2.35.
+template <int KIND>
+__global__ void __launch_bounds__(kRasterWarps * 32, LH_RASTER_MIN_BLOCKS)
+    k_raster(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune, uint32_t list) {
+    __shared__ RasterSmemSmall sm;
+    pdl_enter();
+    phase_raster<KIND>(f, view_begin, n_views, tune, sm, list);
+}
+
+// The occluder pass: a few hundred meshlets, each large on screen.
+__global__ void __launch_bounds__(kRasterWarps * 32, 3)
+    k_raster_occluders(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune) {
     __shared__ RasterSmem sm;
     pdl_enter();
-    phase_raster<KIND, false>(f, view_begin, n_views, tune, &f.status[kStRasterClaim], sm, nullptr, list);
+    phase_raster_general<0, false>(f, view_begin, n_views, tune, sm, nullptr, kListOccluders);
 }
 
 // The alpha-clip draw class (double sided, alpha tested).
 template <int KIND>
-__global__ void __launch_bounds__(kRasterWarps * 32, 3) k_raster_alpha(FrameDev f, uint32_t view_begin,
-                                                                       uint32_t n_views, RasterTune tune, uint32_t list) {
+__global__ void __launch_bounds__(kRasterWarps * 32, 3)
+    k_raster_alpha(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune, uint32_t list) {
     __shared__ RasterSmemAlpha sm;
     pdl_enter();
-    phase_raster<KIND, true>(f, view_begin, n_views, tune, &f.status[kStRasterClaimAlpha], sm, sm.av, list);
+    phase_raster_general<KIND, true>(f, view_begin, n_views, tune, sm, sm.av, list);
 }
 
 template <int KIND>
-__global__ void __launch_bounds__(256, LH_RASTER_BIG_MIN_BLOCKS) k_raster_big(FrameDev f) {
+__global__ void __launch_bounds__(256, LH_RASTER_BIG_MIN_BLOCKS) k_raster_big(const __grid_constant__ FrameDev f) {
+    __shared__ BigSmem sm;
     pdl_enter();
-    phase_raster_big<KIND>(f);
+    phase_raster_big<KIND>(f, sm);
 }
 
 // Hierarchical depth of the visibility views after the occluder pass.
@@ -70,17 +73,13 @@ cudaError_t launch_raster_kind(const FrameDev& f, uint32_t view_begin, uint32_t 
     cudaError_t e;
     if (kind == kViewVisibility) {
         auto opaque = [&](uint32_t list) {
-            if (n_views > 1)
-                return launch_pdl(k_raster<0, LH_RASTER_MULTIVIEW_MIN_BLOCKS>,
-                                  dim3(sms * LH_RASTER_MULTIVIEW_MIN_BLOCKS), rb, s, f, view_begin, n_views, tune, list);
-            return launch_pdl(k_raster<0, LH_RASTER_MIN_BLOCKS>, dim3(sms * LH_RASTER_MIN_BLOCKS), rb, s, f, view_begin,
-                              n_views, tune, list);
+            return launch_pdl(k_raster<0>, dim3(sms * LH_RASTER_MIN_BLOCKS), rb, s, f, view_begin, n_views, tune, list);
         };
         const dim3 big_grid(sms * LH_RASTER_BIG_MIN_BLOCKS);
         if (f.occlusion_px) {
             // occluders (and their chunks), hierarchical depth, the depth
             // test of every other meshlet, then the survivors
-            e = opaque(kListOccluders);
+            e = launch_pdl(k_raster_occluders, dim3(sms * 3), rb, s, f, view_begin, n_views, tune);
             if (e == cudaSuccess) e = launch_pdl(k_raster_big<0>, big_grid, dim3(256), s, f);
             if (e == cudaSuccess) e = launch_pdl(k_hiz, dim3(sms * 4), dim3(256), s, f, view_begin, n_views);
             if (e == cudaSuccess)
@@ -97,8 +96,7 @@ cudaError_t launch_raster_kind(const FrameDev& f, uint32_t view_begin, uint32_t 
         }
         if (e == cudaSuccess) e = launch_pdl(k_raster_big<0>, big_grid, dim3(256), s, f);
     } else {
-        e = launch_pdl(k_raster<1, LH_RASTER_MIN_BLOCKS>, dim3(sms * LH_RASTER_MIN_BLOCKS), rb, s, f, view_begin, n_views,
-                       tune, (uint32_t)kListAll);
+        e = launch_pdl(k_raster<1>, dim3(sms * LH_RASTER_MIN_BLOCKS), rb, s, f, view_begin, n_views, tune, (uint32_t)kListAll);
         if (e == cudaSuccess && f.scene_alpha)
             e = launch_pdl(k_raster_alpha<1>, dim3(sms * 3), rb, s, f, view_begin, n_views, tune, (uint32_t)kListAll);
         if (e == cudaSuccess) e = launch_pdl(k_raster_big<1>, dim3(sms * LH_RASTER_BIG_MIN_BLOCKS), dim3(256), s, f);
