@@ -239,9 +239,11 @@ __device__ void phase_cull_instances_tile(const FrameDev& f, uint32_t view, uint
     __shared__ uint64_t s_warp[kInstTile / 32];
     __shared__ uint64_t s_excl;
     __shared__ uint32_t s_tile;
+    __shared__ SidePlanes s_planes;
     const ViewDev* vw = f.views + view;
     const uint32_t kind = vw->kind, cascade = vw->cascade;
     if (threadIdx.x == 0) s_tile = atomicAdd(&vw->claim[0], 1u);
+    if (kind == kViewVisibility && threadIdx.x == 32) s_planes = side_planes(vw->uniforms->perspective);
     if (kind == kViewVisibility)
         copy_to_smem(&s_u, vw->uniforms, sizeof(Uniforms));
     else
@@ -256,7 +258,7 @@ __device__ void phase_cull_instances_tile(const FrameDev& f, uint32_t view, uint
         load_instance(f.instances + i, ib);
         MeshInfoCull mi = load_mesh_info(mesh_info_of(&ib.inst));
         nm = mi.num_meshlets;
-        keep = kind == kViewVisibility ? !cull_bounding_sphere(s_u, ib.inst.transform, mi.bounding_sphere)
+        keep = kind == kViewVisibility ? !cull_bounding_sphere(s_u.initial_view, s_planes, ib.inst.transform, mi.bounding_sphere)
                                        : !cull_bounding_sphere_shadows(s_m, ib.inst.transform, mi.bounding_sphere, cascade);
     }
     const uint64_t pay = keep ? ((1ull << 40) | nm) : 0ull;
@@ -353,6 +355,7 @@ __device__ void phase_cull_meshlets(const FrameDev& f, uint32_t view_begin, uint
     __shared__ uint32_t s_tile, s_view, s_eab[2], s_tot[2], s_loaded_view;
     __shared__ uint32_t s_tile_off[kMaxViews + 1];
     __shared__ uint64_t s_excl;
+    __shared__ SidePlanes s_planes;
     const uint32_t md = f.max_draws;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -391,6 +394,7 @@ __device__ void phase_cull_meshlets(const FrameDev& f, uint32_t view_begin, uint
         const uint32_t kind = vw->kind, cascade = vw->cascade;
         if (s_loaded_view != v) {
             copy_to_smem(&s_u, vw->uniforms, sizeof(Uniforms));
+            if (threadIdx.x == 64) s_planes = side_planes(vw->uniforms->perspective);
             if (kind == kViewShadow) copy_to_smem(&s_m, f.misc, sizeof(MiscStorage));
         }
         const PrefixSumValue* values = reinterpret_cast<const PrefixSumValue*>(vw->sector + 8);
@@ -444,7 +448,7 @@ __device__ void phase_cull_meshlets(const FrameDev& f, uint32_t view_begin, uint
                 const bool alpha = (mi.flags & MESH_INFO_FLAGS_ALPHA_CLIP) != 0;
                 bool vis;
                 if (kind == kViewVisibility)
-                    vis = !cull_bounding_sphere(s_u, ib.inst.transform, mb.m.bounding_sphere) &&
+                    vis = !cull_bounding_sphere(s_u.initial_view, s_planes, ib.inst.transform, mb.m.bounding_sphere) &&
                           (alpha || !cull_cone_perspective(s_u, &ib.inst, ib.inst.transform, mb.m));
                 else
                     vis = !cull_bounding_sphere_shadows(s_m, ib.inst.transform, mb.m.bounding_sphere, cascade) &&

@@ -68,6 +68,30 @@ __device__ __forceinline__ float gmin(float a, float b) { return (b < a) ? b : a
 __device__ __forceinline__ uint32_t f2u(float f) { return __float_as_uint(f); }
 __device__ __forceinline__ float u2f(uint32_t u) { return __uint_as_float(u); }
 
+// Two floats in a 64-bit register pair: one instruction multiplies or adds
+// both, each rounded on its own (round to nearest even), so a transform's x
+// and y rows (and z and w) take one issue slot per term.  The product is an
+// fma with -0 (the rounded product, its sign kept) whose -0 comes from a
+// kernel parameter: the assembler contracts a packed multiply and the packed
+// add after it into one rounding, whatever the multiply's form, unless it
+// cannot know the addend.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b, f32x2 neg_zero) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(neg_zero));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 // Repeat addressing of texel coordinate i into [0, n): the floor of a
 // sample coordinate below 1e9 in magnitude, so 32 bits hold it.
 __device__ __forceinline__ int32_t wrap_texel(int32_t i, int32_t n) {
@@ -165,25 +189,33 @@ __device__ __forceinline__ MeshInfoResolve load_mesh_info_resolve(const MeshInfo
 
 
 // ------------------------------------------------------------------ culling (culling.glsl)
+// The longest column of the transform's linear part.  The square root is
+// monotone, so the root of the largest square is the largest root, bit for
+// bit (one square root instead of three).
 __device__ __forceinline__ float max_scale(const lh_mat4& t) {
-    float sx = length(f3{t.cols[0].x, t.cols[0].y, t.cols[0].z});
-    float sy = length(f3{t.cols[1].x, t.cols[1].y, t.cols[1].z});
-    float sz = length(f3{t.cols[2].x, t.cols[2].y, t.cols[2].z});
-    return gmax(gmax(sx, sy), sz);
+    auto square = [](const lh_vec4& c) { return dot(f3{c.x, c.y, c.z}, f3{c.x, c.y, c.z}); };
+    return sqrtf(gmax(gmax(square(t.cols[0]), square(t.cols[1])), square(t.cols[2])));
 }
 
-// culling.glsl:1-46; true = culled.
-__device__ __forceinline__ bool cull_bounding_sphere(const Uniforms& u, const lh_mat4& transform, lh_vec4 bs) {
+// culling.glsl:1-46 in two parts: the view's side planes (the same for every
+// sphere of a view: two normalisations, a third of the test's instructions),
+// and the test; true = culled.
+struct SidePlanes {
+    f3 x, y;
+};
+__device__ __forceinline__ SidePlanes side_planes(const lh_mat4& P) {
+    return {normalize(f3{P.cols[0].w + P.cols[0].x, P.cols[1].w + P.cols[1].x, P.cols[2].w + P.cols[2].x}),
+            normalize(f3{P.cols[0].w + P.cols[0].y, P.cols[1].w + P.cols[1].y, P.cols[2].w + P.cols[2].y})};
+}
+__device__ __forceinline__ bool cull_bounding_sphere(const lh_mat4& initial_view, const SidePlanes& f,
+                                                     const lh_mat4& transform, lh_vec4 bs) {
     f4 w4 = mul(transform, f4{bs.x, bs.y, bs.z, 1.0f});
     float radius = bs.w * max_scale(transform);
-    f4 vs = mul(u.initial_view, f4{w4.x, w4.y, w4.z, 1.0f});
+    f4 vs = mul(initial_view, f4{w4.x, w4.y, w4.z, 1.0f});
     vs.z = -vs.z;
     bool visible = vs.z + radius > NEAR_PLANE;
-    const lh_mat4& P = u.perspective;
-    f3 fx = normalize(f3{P.cols[0].w + P.cols[0].x, P.cols[1].w + P.cols[1].x, P.cols[2].w + P.cols[2].x});
-    f3 fy = normalize(f3{P.cols[0].w + P.cols[0].y, P.cols[1].w + P.cols[1].y, P.cols[2].w + P.cols[2].y});
-    visible = visible && vs.z * fx.z + fabsf(vs.x) * fx.x < radius;
-    visible = visible && vs.z * fy.z - fabsf(vs.y) * fy.y < radius;
+    visible = visible && vs.z * f.x.z + fabsf(vs.x) * f.x.x < radius;
+    visible = visible && vs.z * f.y.z - fabsf(vs.y) * f.y.y < radius;
     return !visible;
 }
 

@@ -22,14 +22,18 @@
 //  - every call shares the one array: calls whose work overlaps on the GPU
 //    (different streams, or different host threads) race on it and give
 //    wrong results; serialise them;
-//  - each call clears the array on its own stream before the kernel runs.
+//  - each call clears the array on its own stream before the kernel runs
+//    (calls of at most 4,096 instances run in one cluster and do not use it).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
 #include <mutex>
 
-#include "lh_device.cuh"
-#include "lh_internal.cuh"
+#include "cull_phases.cuh"
+#include "tma.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace lh {
 namespace {
@@ -45,109 +49,151 @@ constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 std::atomic<unsigned long long*> g_scratch_ptr[kMaxDevices];
 
-__device__ __forceinline__ void na_st(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long na_ld(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
 // Same cull and ordered append as the frame's instance cull
 // (cull_instances.comp:7-27 with prefix_sum.glsl:17-30): one instance per
 // thread, warp scans, decoupled look-back with bounded waits.
+//
+// Bound by HBM at the size of an open world (700,001 instances, 78 MB of
+// records: a floor of 12 us).  A tile's records are one bulk copy into shared
+// memory (28 KB, 7 blocks a SM: 200 KB in flight), so no thread's 112-byte
+// stride reaches the memory system, and a record is read from shared memory
+// without bank conflicts (28 words a lane: the 8 lanes of a 16-byte access
+// phase start 4 banks apart).  The look-back reads 32 predecessors at once.
+// 700,001 instances: 43 us, 52 with a thread's loads by itself and a look-back
+// of one predecessor at a time.
 __global__ void __launch_bounds__(kInstTile) k_cull_instances_noalloc(const Instance* instances, uint32_t n,
-                                                                    const Uniforms u, uint8_t* sector,
+                                                                    const __grid_constant__ Uniforms u, uint8_t* sector,
                                                                     uint32_t capacity, uint32_t* flags_out,
                                                                     unsigned long long* scratch) {
-    __shared__ unsigned long long s_warp[kInstTile / 32];
-    __shared__ unsigned long long s_excl;
-    __shared__ uint32_t s_tile;
-    unsigned long long* status = scratch;                         // one word per tile
+    __shared__ __align__(128) Instance s_inst[kInstTile];
+    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ uint64_t s_warp[kInstTile / 32];
+    __shared__ uint64_t s_excl;
+    __shared__ uint32_t s_tile, s_flags;
+    __shared__ SidePlanes s_planes;
+    uint64_t* status = reinterpret_cast<uint64_t*>(scratch);  // one word per tile
     unsigned int* claim = reinterpret_cast<unsigned int*>(scratch + kNoAllocMaxTiles);
-    if (threadIdx.x == 0) s_tile = atomicAdd(claim, 1u);
+    if (threadIdx.x == 0) {
+        mbar_init(&s_bar, 1);
+        mbar_init_fence();
+        const uint32_t tile = atomicAdd(claim, 1u);
+        s_tile = tile;
+        s_flags = 0u;
+        if (tile < gridDim.x) {
+            const uint32_t bytes = min(n - tile * kInstTile, kInstTile) * (uint32_t)sizeof(Instance);
+            mbar_expect_tx(&s_bar, bytes);
+            bulk_load(s_inst, instances + (size_t)tile * kInstTile, bytes, &s_bar);
+        }
+        s_planes = side_planes(u.perspective);
+    }
     __syncthreads();
     const uint32_t tile = s_tile;
+    if (tile >= gridDim.x) return;  // another call's claims: wrong results, but none out of range
     const uint32_t i = tile * kInstTile + threadIdx.x;
+    // (a copy that never lands: reported, the tile counts as empty)
+    const bool landed = mbar_wait(&s_bar, 0u);
+    if (!landed) atomicOr(&s_flags, LH_FLAG_TIMEOUT);
     bool keep = false;
+    uint32_t nm = 0;
+    if (landed && i < n) {
+        const Instance& inst = s_inst[threadIdx.x];
+        const MeshInfoCull mi = load_mesh_info(mesh_info_of(&inst));
+        nm = mi.num_meshlets;
+        keep = !cull_bounding_sphere(u.initial_view, s_planes, inst.transform, mi.bounding_sphere);
+    }
+    const uint64_t pay = keep ? ((1ull << 40) | nm) : 0ull;
+    const uint64_t incl = warp_incl_scan(pay);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        uint64_t sum = lane < kInstTile / 32 ? s_warp[lane] : 0ull;
+        const uint64_t own = sum;
+        sum = warp_incl_scan(sum);
+        if (lane < kInstTile / 32) s_warp[lane] = sum - own;
+        const uint64_t run = __shfl_sync(0xFFFFFFFFu, sum, kInstTile / 32 - 1);
+        const uint64_t excl = lookback_warp(status, tile, run, &s_flags);
+        if (lane == 0) {
+            s_excl = excl;
+            if (tile == gridDim.x - 1) {
+                const uint64_t total = excl + run, count = total >> 40;
+                *reinterpret_cast<unsigned long long*>(sector) = (count << 32) | (uint32_t)(total & kSum40);
+                if (count > capacity) s_flags |= LH_FLAG_INSTANCE_OVERFLOW;
+            }
+            if (s_flags && flags_out) atomicOr(flags_out, s_flags);
+        }
+    }
+    __syncthreads();
+    if (keep) {
+        const uint64_t before = s_excl + s_warp[warp] + incl - pay;
+        const uint32_t pos = (uint32_t)(before >> 40);
+        if (pos < capacity) {
+            PrefixSumValue v;
+            v.index = i;
+            v.sum = (uint32_t)(before & kSum40) + nm;
+            reinterpret_cast<PrefixSumValue*>(sector + 8)[pos] = v;
+        }
+    }
+    if (!landed) mbar_wait(&s_bar, 0u);  // the block does not leave a copy behind
+}
+
+// The same for at most kSmallInstances instances, by one cluster: its blocks
+// pass their totals through shared memory, so nothing has to be cleared first and
+// the call is one launch.  Bound by latency and, at one block, by issue (the
+// square roots and divisions of 32 warps on one SM): inside a graph 1,024
+// instances take 2.3 us by 8 blocks, 4.1 by one, 4.4 cleared and by tiles; 4,096
+// take 3.6 and 4,097, by tiles, 5.1.  A call by itself: 4.1 us, 9.2 before.
+constexpr uint32_t kSmallBlocks = 8, kSmallThreads = 512, kSmallInstances = kSmallBlocks * kSmallThreads;
+__global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads) k_cull_instances_noalloc_small(
+    const Instance* instances, uint32_t n, const __grid_constant__ Uniforms u, uint8_t* sector, uint32_t capacity,
+    uint32_t* flags_out) {
+    __shared__ uint64_t s_warp[kSmallThreads / 32];
+    __shared__ uint64_t s_block[kSmallBlocks];
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.barrier_arrive();  // waited for before the first access to another block's memory
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = blockIdx.x;
+    const uint32_t i = rank * blockDim.x + threadIdx.x;
+    uint64_t pay = 0;
     uint32_t nm = 0;
     if (i < n) {
         const Instance* inst = instances + i;
         lh_mat4 transform;
         const float4* src = reinterpret_cast<const float4*>(inst);
         float4* dst = reinterpret_cast<float4*>(&transform);
-        for (int k = 0; k < 4; k++) dst[k] = __ldg(src + k);
-        const MeshInfo* mi = mesh_info_of(inst);
-        const unsigned long long* w = reinterpret_cast<const unsigned long long*>(mi);
-        unsigned long long w6 = __ldg(w + 6), w7 = __ldg(w + 7);
-        lh_vec4 bs;
-        bs.x = __uint_as_float((uint32_t)(w6 >> 32));
-        bs.y = __uint_as_float((uint32_t)w7);
-        bs.z = __uint_as_float((uint32_t)(w7 >> 32));
-        bs.w = __uint_as_float(__ldg(reinterpret_cast<const uint32_t*>(mi) + 16));
-        nm = (uint32_t)(w6 & 0xFFFFu);
-        keep = !cull_bounding_sphere(u, transform, bs);
+#pragma unroll
+        for (int c = 0; c < 4; c++) dst[c] = __ldg(src + c);
+        const MeshInfoCull mi = load_mesh_info(mesh_info_of(inst));
+        nm = mi.num_meshlets;
+        if (!cull_bounding_sphere(u.initial_view, side_planes(u.perspective), transform, mi.bounding_sphere))
+            pay = (1ull << 40) | nm;
     }
-    const unsigned long long pay = keep ? ((1ull << 40) | nm) : 0ull;
-    unsigned long long incl = pay;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= (uint32_t)o) incl += v;
-    }
+    const uint64_t incl = warp_incl_scan(pay);
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long run = 0;
-        for (uint32_t k = 0; k < kInstTile / 32; k++) {
-            unsigned long long t = s_warp[k];
-            s_warp[k] = run;
-            run += t;
-        }
-        unsigned long long excl = 0;
-        if (tile == 0) {
-            na_st(&status[0], kStatIncl | run);
-        } else {
-            na_st(&status[tile], kStatAgg | run);
-            int64_t t = (int64_t)tile - 1;
-            uint32_t spins = 0;
-            while (t >= 0) {
-                unsigned long long s = na_ld(&status[t]);
-                unsigned long long fl = s >> 62;
-                if (fl == 0) {
-                    if (++spins >= kSpinLimit) {
-                        // recorded by the block that timed out, whenever it does
-                        if (flags_out) atomicOr(flags_out, LH_FLAG_TIMEOUT);
-                        break;
-                    }
-                    if (spins > 32) __nanosleep(spins > 1024 ? 256 : 32);
-                    continue;
-                }
-                excl += s & kPayloadMask;
-                if (fl == 2) break;
-                --t;
-            }
-            na_st(&status[tile], kStatIncl | (excl + run));
-        }
-        s_excl = excl;
-        if (tile == gridDim.x - 1) {
-            unsigned long long total = excl + run;
-            unsigned long long count = total >> 40;
-            *reinterpret_cast<unsigned long long*>(sector) = (count << 32) | (uint32_t)(total & ((1ull << 40) - 1));
-            if (count > capacity) {
-                if (flags_out) atomicOr(flags_out, LH_FLAG_INSTANCE_OVERFLOW);
-            }
-        }
+    const uint64_t sums = warp_incl_scan(lane < blockDim.x / 32 ? s_warp[lane] : 0ull);
+    const uint64_t own = __shfl_sync(0xffffffffu, sums, 31);
+    uint64_t before = __shfl_sync(0xffffffffu, sums, warp ? warp - 1 : 0);
+    before = (warp ? before : 0) + incl - pay;
+    cluster.barrier_wait();
+    if (threadIdx.x < kSmallBlocks) *cluster.map_shared_rank(&s_block[rank], threadIdx.x) = own;
+    cluster.sync();
+    uint64_t total = 0;
+#pragma unroll
+    for (uint32_t b = 0; b < kSmallBlocks; b++) {
+        if (b == rank) before += total;
+        total += s_block[b];
     }
-    __syncthreads();
-    if (keep) {
-        unsigned long long before = s_excl + s_warp[warp] + incl - pay;
-        uint32_t pos = (uint32_t)(before >> 40);
+    if (rank == 0 && threadIdx.x == 0) {
+        const uint64_t count = total >> 40;
+        *reinterpret_cast<unsigned long long*>(sector) = (count << 32) | (uint32_t)(total & kSum40);
+        if (count > capacity && flags_out) atomicOr(flags_out, LH_FLAG_INSTANCE_OVERFLOW);
+    }
+    if (pay) {
+        const uint32_t pos = (uint32_t)(before >> 40);
         if (pos < capacity) {
             PrefixSumValue v;
             v.index = i;
-            v.sum = (uint32_t)(before & ((1ull << 40) - 1)) + nm;
+            v.sum = (uint32_t)(before & kSum40) + nm;
             reinterpret_cast<PrefixSumValue*>(sector + 8)[pos] = v;
         }
     }
@@ -193,6 +239,12 @@ extern "C" lh_status lh_cull_instances_noalloc(const Instance* d_instances, uint
     unsigned long long* scratch = nullptr;
     lh_status st = scratch_for_current_device(s, &scratch);
     if (st != LH_OK) return st;
+    if (n_instances && n_instances <= kSmallInstances) {
+        const uint32_t per_block = (n_instances + kSmallBlocks - 1) / kSmallBlocks;
+        k_cull_instances_noalloc_small<<<kSmallBlocks, (per_block + 31) & ~31u, 0, s>>>(
+            d_instances, n_instances, *host_uniforms, d_sector, capacity, d_flags);
+        return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ERR_CUDA;
+    }
     // the previous call's look-back words and claim counter must not leak in
     if (cudaMemsetAsync(scratch, 0, sizeof(unsigned long long) * kNoAllocWords, s) != cudaSuccess) return LH_ERR_CUDA;
     if (tiles == 0) {

@@ -731,30 +731,6 @@ __device__ __forceinline__ void raster_meshlet(const FrameDev& f, const MeshletW
     __syncwarp();
 }
 
-// Two floats in a 64-bit register pair: one instruction multiplies or adds
-// both, each rounded on its own (round to nearest even), so a transform's x
-// and y rows (and z and w) take one issue slot per term.  The product is an
-// fma with -0 (the rounded product, its sign kept) whose -0 comes from a
-// kernel parameter: the assembler contracts a packed multiply and the packed
-// add after it into one rounding, whatever the multiply's form, unless it
-// cannot know the addend.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b, f32x2 neg_zero) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(neg_zero));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 // A column-major matrix as row pairs: xy[c], zw[c] of column c.
 struct Mat2 {
     f32x2 xy[4], zw[4];

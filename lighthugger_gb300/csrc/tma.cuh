@@ -55,6 +55,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 
+// Untiled bulk copy of `bytes` from global `src` into shared memory `dst`,
+// completing on `bar`: both addresses 16-byte aligned, the size a multiple of
+// 16 bytes.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 // 2D tiled load of box (x, y) of `map` into shared memory `dst`, completing
 // on `bar`.  x * element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int32_t x, int32_t y, uint64_t* bar) {
