@@ -5,8 +5,18 @@
 // gradients into the caller's buffers.  Targets every lane of a warp shares
 // (light direction / colour, a material's base-colour factor) are summed
 // across the warp first, so they take one atomic per warp.
+//
+// Bound by instruction issue and the latency of its gathers at 16 warps an
+// SM (128 registers; 24 warps at 80 spill and take 760 us).  Every pixel by
+// itself: triangles are small where it matters (15 distinct ones in a row of
+// 32 pixels in the 1080p scene seen from above; records shared by a warp's
+// pixels, 8 to 16 triangles at a time, took 4 times as long).  The gradients
+// of slivers are ill-conditioned, so a pixel's arithmetic keeps its order
+// and rounding.  That scene: 505 us with the triangle's terms formed three
+// times a pixel and four looks at the runs per texture sample, 405 now.
 #include <algorithm>
 
+#include "exact_div.cuh"
 #include "frame_phases.cuh"
 #include "shade.cuh"
 #include "tma.cuh"
@@ -42,12 +52,13 @@ struct DeviceSampler {
         s.b = v - fv;
         const int32_t i0 = (int32_t)fu, j0 = (int32_t)fv;
         const int32_t W = (int32_t)t.width, H = (int32_t)t.height;
-        s.i0 = wrap_texel(i0, W);
-        s.i1 = wrap_texel(i0 + 1, W);
-        s.j0 = wrap_texel(j0, H);
-        s.j1 = wrap_texel(j0 + 1, H);
         s.size_u = (float)t.width;
         s.size_v = (float)t.height;
+        // i0 + 1 wraps to the texel after i0's (or 0 past the last)
+        s.i0 = wrap_texel(i0, W);
+        s.i1 = s.i0 + 1 == W ? 0 : s.i0 + 1;
+        s.j0 = wrap_texel(j0, H);
+        s.j1 = s.j0 + 1 == H ? 0 : s.j0 + 1;
         auto texel = [&](int32_t i, int32_t j, float* o) {
             const float4 p = __ldg(tex + ((size_t)j * W + i));
             o[0] = p.x;
@@ -69,6 +80,23 @@ struct DeviceSampler {
     }
 };
 
+// The 4 x 4 window inside the map: no clamping (compare_window of shade.cuh).
+__device__ uint32_t compare_window(const DeviceSampler& smp, uint32_t layer, int32_t i, int32_t j, float ref) {
+    const int32_t S = (int32_t)smp.f->shadow_size;
+    uint32_t win = 0;
+    if (i >= 0 && j >= 0 && i <= S - 4 && j <= S - 4) {
+        const float* row = smp.f->shadow_maps + ((size_t)layer * S + j) * S + i;
+#pragma unroll
+        for (int r = 0; r < 4; r++, row += S)
+#pragma unroll
+            for (int c = 0; c < 4; c++) win |= (ref < __ldg(row + c) ? 1u : 0u) << (4 * r + c);
+        return win;
+    }
+#pragma unroll 1
+    for (int k = 0; k < 16; k++) win |= (smp.shadow_cmp(layer, i + (k & 3), j + (k >> 2), ref) != 0.0f ? 1u : 0u) << k;
+    return win;
+}
+
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 // Launch shape: tiles of 32 x ROWS pixels (ROWS = 4, 8 or 16, chosen at run
 // time through lh_tuning.backward_rows), one warp per row, and the threads
@@ -80,31 +108,74 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint32_t kCacheSlots = 256;     // shared-memory accumulators of hot gradient addresses
 constexpr uint32_t kSmallTexture = 64;    // textures of at most this many texels go through them
 
-// Fixed inputs of a pixel for shade.cuh whose matrices are read from
-// memory at each use -- PV and the cascades' UVS from the block's shared
-// copies, the instance's normal transform from global memory -- rather
-// than held in registers through the whole pixel.  `pv3` / `uvs3` point at
-// the column 3 in use (absolute for the decisions, camera-relative after).
-__device__ __forceinline__ float lds_f32(const float* p) {
+// Shared-memory reads that the compiler neither merges nor moves: a value is
+// read where it is used instead of held in a register through the pixel.
+__device__ __forceinline__ float lds_f32(uint32_t a) {
     float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(smem_u32(p)));
-    return v;
-}
-__device__ __forceinline__ float ldg_f32(const float* p) {
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
     return v;
 }
 
+// The terms of a pixel's triangle (shade.cuh's TriTerms and the instance's
+// normal transform) in the thread's own column of shared memory, word j of
+// the warp's 32 threads side by side.  They serve the forward and both parts
+// of the reverse, each computed once: in registers they would not last
+// through the BRDF, and recomputed where they are used they were a fifth of
+// the kernel's instructions.
+enum : uint32_t {
+    kTermW = 0,        // 9: camera-relative positions
+    kTermN = 9,        // 9: normalised normals
+    kTermRn = 18,      // 3: 1 / length of the raw normals
+    kTermC = 21,       // 6: clip x, y
+    kTermIw = 27,      // 3: 1 / clip w
+    kTermProj = 30,    // 6: projected x, y
+    kTermSlope = 36,   // 6: slopes of lambda / w
+    kTermSum = 42,     // 2: their sums
+    kTermInvDet = 44,  // 1
+    kTermUv = 45,      // 6: uvs times the texture scale
+    kTermTs = 51,      // 2: texture scale
+    kTermToff = 53,    // 2: texture offset
+    kTermNt = 55,      // 9: normal transform
+    kTerms = 64
+};
+struct ThreadTri {
+    uint32_t at;  // shared-memory address of the thread's word 0
+    __device__ float get(uint32_t j) const { return lds_f32(at + 128 * j); }
+    __device__ void set(uint32_t j, float v) const { asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 128 * j), "f"(v)); }
+    __device__ v2<float> get2(uint32_t j) const { return {get(j), get(j + 1)}; }
+    __device__ v3<float> get3(uint32_t j) const { return {get(j), get(j + 1), get(j + 2)}; }
+    __device__ void set2(uint32_t j, v2<float> v) const { set(j, v.x), set(j + 1, v.y); }
+    __device__ void set3(uint32_t j, v3<float> v) const { set(j, v.x), set(j + 1, v.y), set(j + 2, v.z); }
+    __device__ v3<float> W(int k) const { return get3(kTermW + 3 * k); }
+    __device__ v3<float> nk(int k) const { return get3(kTermN + 3 * k); }
+    __device__ float rn(int k) const { return get(kTermRn + k); }
+    __device__ v2<float> C(int k) const { return get2(kTermC + 2 * k); }
+    __device__ float iw(int k) const { return get(kTermIw + k); }
+    __device__ v2<float> n(int k) const { return get2(kTermProj + 2 * k); }
+    __device__ v2<float> dd(int k) const { return get2(kTermSlope + 2 * k); }
+    __device__ v2<float> s() const { return get2(kTermSum); }
+    __device__ float inv_det() const { return get(kTermInvDet); }
+    __device__ v2<float> uvs(int k) const { return get2(kTermUv + 2 * k); }
+    __device__ v2<float> ts() const { return get2(kTermTs); }
+    __device__ v2<float> toff() const { return get2(kTermToff); }
+};
+
+// Fixed inputs of a pixel for shade.cuh; its matrices are read from shared
+// memory at each use: PV and the cascade's UVS, camera-relative, from the
+// block's copies, the normal transform from the thread's terms.  `uvs3`
+// points at the column 3 in use (absolute for the decisions).
 struct DeviceFixed : shade::PixelScalars {
-    const float* pv;    // shared: 16 floats, column-major
-    const float* pv3;   // shared: 4 floats
-    const float* uvs;   // shared: 16 floats of the pixel's cascade
-    const float* uvs3;  // shared: 4 floats
-    const float* nt;    // global: Instance::normal_transform, 3 columns of 3
-    __device__ float PV(int c, int r) const { return c == 3 ? lds_f32(pv3 + r) : lds_f32(pv + 4 * c + r); }
-    __device__ float UVS(int c, int r) const { return c == 3 ? lds_f32(uvs3 + r) : lds_f32(uvs + 4 * c + r); }
-    __device__ float NT(int c, int r) const { return ldg_f32(nt + 3 * c + r); }
+    uint32_t pv;         // 16 floats, column-major
+    uint32_t uvs, uvs3;  // 16 floats of the pixel's cascade; 4 floats
+    uint32_t nt;         // 9 words of the thread's
+    __device__ float PV(int c, int r) const { return lds_f32(pv + 16 * c + 4 * r); }
+    __device__ float UVS(int c, int r) const { return lds_f32((c == 3 ? uvs3 : uvs + 16 * c) + 4 * r); }
+    __device__ float NT(int c, int r) const { return lds_f32(nt + 128 * (3 * c + r)); }
+};
+// The same with PV in registers, for the transforms of the three vertices.
+struct VertexFixed : shade::PixelScalars {
+    const float *pv, *pv3;  // shared
+    __device__ float PV(int c, int r) const { return c == 3 ? pv3[r] : pv[4 * c + r]; }
 };
 
 // Block-shared copies of the frame's matrices for DeviceFixed.
@@ -195,13 +266,24 @@ struct PixelOut {
     uint32_t idx[3];
 };
 
+// sign(dot(gn, normalize(vd))) as the IEEE arithmetic of the forward gives
+// it.  Its rounding moves the dot product by less than 2^-21 of the sum of
+// the terms' magnitudes and the undivided one's by less than 2^-22, so only
+// a sum of nearly cancelling terms (or of extreme ones) needs the divisions.
+__device__ __forceinline__ bool faces_away(f3 gn, f3 vd) {
+    const float x = gn.x * vd.x, y = gn.y * vd.y, z = gn.z * vd.z, d2 = dot(vd, vd);
+    const float s = (x + y) + z, m = (fabsf(x) + fabsf(y)) + fabsf(z);
+    if (fabsf(s) > m * (1.0f / 262144.0f) && fabsf(s) > 1e-30f && d2 > 1e-20f && d2 < 1e12f) return s < 0.0f;
+    return dot(gn, normalize(vd)) < 0.0f;
+}
+
 // Recompute the forward of pixel (x, y) from the visibility buffer and run
 // the surface half of the reverse pass of shade.cuh for the upstream
-// gradient at that pixel; fx, p and st carry what the geometry half needs.
+// gradient at that pixel; fx, tri and st carry what the geometry half needs.
 // `M` holds the block's copies of the frame matrices.
 __device__ __forceinline__ void pixel_backward(const FrameDev& f, const float4* grad, const lh_grad_targets& t,
-                                               const FrameMats& M, uint32_t x, uint32_t y, PixelGrad<float>& g,
-                                               PixelOut& o, DeviceFixed& fx, PixelParams<float>& p,
+                                               const FrameMats& M, uint32_t x, uint32_t y, float rcp_w,
+                                               PixelGrad<float>& g, PixelOut& o, DeviceFixed& fx, const ThreadTri& tri,
                                                shade::SurfaceState<float>& st) {
     const Uniforms& u = *f.uniforms;
     const uint32_t W = u.window_size.x, H = u.window_size.y;
@@ -211,23 +293,27 @@ __device__ __forceinline__ void pixel_backward(const FrameDev& f, const float4* 
     if (active) vis = __ldcs(reinterpret_cast<const unsigned long long*>(f.visibility) + (size_t)y * W + x);
     active = active && u2f((uint32_t)(vis >> 32)) != 0.0f;
     if (!active) return;
-    const float4 gp = __ldcs(grad + (size_t)y * W + x);
     const uint32_t packed = (uint32_t)vis;
-    const uint32_t slot = packed & ((1u << 24) - 1u), tri = packed >> 24;
+    const uint32_t slot = packed & ((1u << 24) - 1u), tri_index = packed >> 24;
     // the slot's draw record (written by the meshlet cull): the instance and
     // the index / micro-index addresses already offset to the meshlet, so
     // the vertex loads do not wait on the reference, MeshInfo and Meshlet
     const RasterDraw rd = f.views[0].rdraws[slot];
     const Instance* inst = f.instances + rd.instance;
     const MeshInfoResolve mi = load_mesh_info_resolve(mesh_info_of(inst));
-    const uint8_t* micro = reinterpret_cast<const uint8_t*>(rd.micro) + tri * 3;
+    if (mi.normal_tex != UNUSED_TEXTURE_INDEX) return;  // normal-mapped: not differentiated
+    const float4 gp = __ldcs(grad + (size_t)y * W + x);
+    const uint8_t* micro = reinterpret_cast<const uint8_t*>(rd.micro) + tri_index * 3;
     const uint32_t flags = mi.flags;
+#pragma unroll
     for (int k = 0; k < 3; k++) {
         const uint32_t vi = __ldg(micro + k);
         o.idx[k] = (flags & MESH_INFO_FLAGS_32_BIT_INDICES) ? __ldg(reinterpret_cast<const uint32_t*>(rd.indices) + vi)
                                                             : __ldg(reinterpret_cast<const uint16_t*>(rd.indices) + vi);
     }
+    PixelParams<float> p;
     const lh_mat4& T = inst->transform;
+#pragma unroll
     for (int k = 0; k < 3; k++) {
         f3 w = world_pos(T, load_position(rd.positions, flags, o.idx[k]));
         p.W[k] = {w.x, w.y, w.z};
@@ -239,33 +325,29 @@ __device__ __forceinline__ void pixel_backward(const FrameDev& f, const float4* 
     p.bcf = {mi.base_color_factor.x, mi.base_color_factor.y, mi.base_color_factor.z};
     p.sun = {u.sun_dir.x, u.sun_dir.y, u.sun_dir.z};
     p.light = {u.sun_intensity.x, u.sun_intensity.y, u.sun_intensity.z};
-    fx.pv = M.pv;
-    fx.pv3 = M.pv + 12;
-    fx.nt = &inst->normal_transform.cols[0].x;
-    const f2 ndc{(float)x / (float)W * 2.0f - 1.0f, (float)y / (float)H * 2.0f - 1.0f};
-    fx.ndc[0] = ndc.x;
-    fx.ndc[1] = ndc.y;
-    fx.win[0] = (float)W;
-    fx.win[1] = (float)H;
-    fx.cam[0] = u.camera_pos.x;
-    fx.cam[1] = u.camera_pos.y;
-    fx.cam[2] = u.camera_pos.z;
-    fx.ts[0] = mi.texture_scale.x;
-    fx.ts[1] = mi.texture_scale.y;
-    fx.toff[0] = mi.texture_offset.x;
-    fx.toff[1] = mi.texture_offset.y;
+    // x / W * 2 - 1 with the quotient from the reciprocal (the same bits)
+    const float qx = W <= (uint32_t)kExactDivMaxCount ? div_by_count((float)x, (float)W, rcp_w) : (float)x / (float)W;
+    VertexFixed vx;
+    vx.pv = M.pv;
+    vx.pv3 = M.pv + 12;
+    vx.ndc[0] = fx.ndc[0] = qx * 2.0f - 1.0f;
+    vx.ndc[1] = fx.ndc[1] = (float)y / (float)H * 2.0f - 1.0f;
+    vx.ts[0] = mi.texture_scale.x;
+    vx.ts[1] = mi.texture_scale.y;
+    vx.toff[0] = mi.texture_offset.x;
+    vx.toff[1] = mi.texture_offset.y;
     fx.thin = (flags & MESH_INFO_FLAGS_ALPHA_CLIP) ? 1u : 0u;
     fx.bias = fx.thin ? 0.000002f : 0.0f;
     fx.shadow_size = (float)f.shadow_size;
     fx.base_tex = mi.base_tex;
     fx.mr_tex = mi.mr_tex;
-    fx.has_normal_map = mi.normal_tex != UNUSED_TEXTURE_INDEX;
+    fx.has_normal_map = 0u;
     DeviceSampler smp{&f};
     {
         // the world position the forward interpolated, in its absolute float
         // arithmetic, picks the cascade (render_geometry.comp:183-196) and
         // places the PCF taps
-        const v3<float> world = shade::forward_world(fx, p);
+        const v3<float> world = shade::forward_world(vx, p);
         uint32_t ci;
         for (ci = 0; ci < 4; ci++) {
             const lh_mat4& m = *reinterpret_cast<const lh_mat4*>(M.uvs[ci]);
@@ -274,21 +356,46 @@ __device__ __forceinline__ void pixel_backward(const FrameDev& f, const float4* 
             if (fabsf(ox) < 0.5f && fabsf(oy) < 0.5f) break;
         }
         fx.cascade = ci;
-        fx.uvs = M.uvs[ci > 3 ? 3 : ci];
-        fx.uvs3 = fx.uvs + 12;
+        fx.uvs = smem_u32(M.uvs[ci > 3 ? 3 : ci]);
+        fx.uvs3 = fx.uvs + 48;
         // face flip, far-plane test and compare results exactly as the forward
-        shade::decide_at(fx, p, world, smp);
+        const f3 a{p.W[0].x, p.W[0].y, p.W[0].z}, b{p.W[1].x, p.W[1].y, p.W[1].z}, c{p.W[2].x, p.W[2].y, p.W[2].z};
+        fx.flip = faces_away(cross(b - a, c - a), ld3(u.camera_pos) - f3{world.x, world.y, world.z}) ? -1.0f : 1.0f;
+        shade::decide_shadow(fx, world, smp);
     }
     // the continuous part in camera-relative coordinates: W - cam is
     // (nearly) exact, and PV T(cam), UVS T(cam) were formed in double
     const uint32_t layer = fx.cascade > 3 ? 3u : fx.cascade;
-    fx.pv3 = M.rel;
-    fx.uvs3 = M.rel + 4 + 4 * layer;
-    for (int k = 0; k < 3; k++) p.W[k] = {p.W[k].x - u.camera_pos.x, p.W[k].y - u.camera_pos.y, p.W[k].z - u.camera_pos.z};
+    fx.uvs3 = smem_u32(M.rel + 4 + 4 * layer);
+    fx.pv = smem_u32(M.pv);
+    fx.nt = tri.at + 128 * kTermNt;
     fx.cam[0] = fx.cam[1] = fx.cam[2] = 0.0f;
+    {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            p.W[k] = {p.W[k].x - u.camera_pos.x, p.W[k].y - u.camera_pos.y, p.W[k].z - u.camera_pos.z};
+        vx.pv3 = M.rel;
+        const shade::TriTerms<float> terms = shade::tri_terms(vx, p);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            tri.set3(kTermW + 3 * k, terms.w_[k]);
+            tri.set3(kTermN + 3 * k, terms.nk_[k]);
+            tri.set(kTermRn + k, terms.rn_[k]);
+            tri.set2(kTermC + 2 * k, terms.c_[k]);
+            tri.set(kTermIw + k, terms.iw_[k]);
+            tri.set2(kTermProj + 2 * k, terms.n_[k]);
+            tri.set2(kTermSlope + 2 * k, terms.dd_[k]);
+            tri.set2(kTermUv + 2 * k, terms.uvs_[k]);
+            const lh_vec3& nt = inst->normal_transform.cols[k];
+            tri.set3(kTermNt + 3 * k, v3<float>{nt.x, nt.y, nt.z});
+        }
+        tri.set2(kTermSum, terms.s_);
+        tri.set(kTermInvDet, terms.inv_det_);
+        tri.set2(kTermTs, terms.ts_);
+        tri.set2(kTermToff, terms.toff_);
+    }
     v3<float> out;
-    shade::shade_surface<float>(fx, p, smp, &out, v3<float>{gp.x, gp.y, gp.z}, &g, &st);
-    if (!g.differentiated) return;
+    shade::shade_surface<float>(fx, p, tri, smp, &out, v3<float>{gp.x, gp.y, gp.z}, &g, &st);
     o.ok = true;
     o.packed = packed;
     o.inst = inst;
@@ -297,51 +404,68 @@ __device__ __forceinline__ void pixel_backward(const FrameDev& f, const float4* 
                              : nullptr;
 }
 
-// The four texels of one bilinear sample (00, 10, 01, 11): run-summed along
-// the warp and added to the texture's gradient image, channels [c0, c0 + nc).
-// Taps that land on the same texel (1-texel-wide textures, edges) are merged
-// into the first.
+// The four texels of one bilinear sample (00, 10, 01, 11): summed over the
+// run of pixels along the warp that sample the same four, and added to the
+// texture's gradient image, channels [c0, c0 + NC).  Equal first texels of
+// one texture have equal others, so one look at the runs serves all four
+// (each by itself: 120 us of the kernel's 470 at 1920 x 1080, 74 so).  In a
+// texture one texel wide or high, taps on the same texel are merged.
 template <int NC>
-__device__ __forceinline__ void scatter_texels(HotCache& cache, float* const base_addr[4], float v[4][NC], int c0,
-                                               bool small) {
-    float* a[4] = {base_addr[0], base_addr[1], base_addr[2], base_addr[3]};
+__device__ __forceinline__ void scatter_texels(HotCache& cache, float* dst, const lh_texture& t, const int32_t ij[4],
+                                               float v[4][NC], int c0) {
+    const int32_t W = dst ? (int32_t)t.width : 0;
+    float* const first = dst ? dst + 4 * ((size_t)ij[2] * W + ij[0]) : nullptr;
+    if (!__any_sync(kFull, first != nullptr)) return;
+    const Run r = run_of((unsigned long long)first);
+    if (r.span > 1) {
+        float s[4 * NC];
 #pragma unroll
-    for (int q = 1; q < 4; q++)
+        for (int q = 0; q < 4; q++)
 #pragma unroll
-        for (int p = 0; p < q; p++)
-            if (a[q] && a[q] == a[p]) {
+            for (int c = 0; c < NC; c++) s[q * NC + c] = v[q][c];
+        run_sums(s, r);
 #pragma unroll
-                for (int c = 0; c < NC; c++) {
-                    v[p][c] += v[q][c];
-                    v[q][c] = 0.0f;
-                }
-                a[q] = nullptr;
-            }
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) v[q][c] = s[q * NC + c];
+    }
+    if (!r.head || !first) return;
+    const bool one_wide = ij[0] == ij[1], one_high = ij[2] == ij[3];
+    if (one_wide || one_high) {
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            if (one_wide) v[0][c] += v[1][c], v[2][c] += v[3][c];
+            if (one_high) v[0][c] += v[2][c], v[1][c] += v[3][c];
+        }
+    }
+    const bool small = t.width * t.height <= kSmallTexture;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        if (!__any_sync(kFull, a[q] != nullptr)) continue;
-        const Run r = run_of((unsigned long long)a[q]);
-        float s[NC];
+        if (((q & 1) && one_wide) || ((q >> 1) && one_high)) continue;
+        float* a = dst + 4 * ((size_t)ij[2 + (q >> 1)] * W + ij[q & 1]);
+        if (!small && ((uintptr_t)a & 15u) == 0) {
+            // one vector reduction per texel (the other channels add 0)
+            float4 d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            float* dc = &d.x;
 #pragma unroll
-        for (int c = 0; c < NC; c++) s[c] = v[q][c];
-        run_sums(s, r);
-        if (r.head && a[q]) {
-            if (!small && ((uintptr_t)a[q] & 15u) == 0) {
-                // one vector reduction per texel (the other channels add 0)
-                float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                float* tc = &t.x;
+            for (int c = 0; c < NC; c++) dc[c0 + c] = v[q][c];
+            atomicAdd(reinterpret_cast<float4*>(a), d);
+        } else {
 #pragma unroll
-                for (int c = 0; c < NC; c++) tc[c0 + c] = s[c];
-                atomicAdd(reinterpret_cast<float4*>(a[q]), t);
-            } else {
-#pragma unroll
-                for (int c = 0; c < NC; c++) {
-                    if (small) cache_add(cache, a[q] + c0 + c, s[c]);
-                    else atomicAdd(a[q] + c0 + c, s[c]);
-                }
+            for (int c = 0; c < NC; c++) {
+                if (small) cache_add(cache, a + c0 + c, v[q][c]);
+                else atomicAdd(a + c0 + c, v[q][c]);
             }
         }
     }
+}
+
+// Three neighbouring floats: a pair and a single, the pair where it is
+// aligned to 8 bytes.
+__device__ __forceinline__ void add3(float* p, f3 v) {
+    const bool even = ((uintptr_t)p & 7u) == 0;
+    atomicAdd(reinterpret_cast<float2*>(even ? p : p + 1), even ? make_float2(v.x, v.y) : make_float2(v.y, v.z));
+    atomicAdd(even ? p + 2 : p, even ? v.z : v.x);
 }
 
 // Column 3 of PV T(cam) and of UVS_c T(cam) for the 4 cascades, in double
@@ -372,6 +496,7 @@ __global__ void __launch_bounds__(32 * ROWS, LH_BWD_MIN_BLOCKS * 8 / ROWS)
     __shared__ float s_light[ROWS][6];
     pdl_enter();
     __shared__ __align__(16) FrameMats s_mats;
+    extern __shared__ __align__(16) float s_terms[];  // [ROWS][kTerms][32]
     const uint32_t tid = threadIdx.y * 32 + threadIdx.x;
     for (uint32_t s = tid; s < kCacheSlots; s += 32 * ROWS) {
         cache.key[s] = 0ull;
@@ -383,14 +508,15 @@ __global__ void __launch_bounds__(32 * ROWS, LH_BWD_MIN_BLOCKS * 8 / ROWS)
     __syncthreads();
     float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     const uint64_t* tex_targets = reinterpret_cast<const uint64_t*>(t.texture_grads);
+    const ThreadTri tri{smem_u32(s_terms + threadIdx.y * (kTerms * 32) + threadIdx.x)};
+    const float rcp_w = 1.0f / (float)f.uniforms->window_size.x;
     for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const uint32_t x = (tile % tiles_x) * 32 + threadIdx.x, y = (tile / tiles_x) * ROWS + threadIdx.y;
         PixelGrad<float> g;
         PixelOut o;
         DeviceFixed fx;
-        PixelParams<float> p;
         shade::SurfaceState<float> st;
-        pixel_backward(f, grad, t, s_mats, x, y, g, o, fx, p, st);
+        pixel_backward(f, grad, t, s_mats, x, y, rcp_w, g, o, fx, tri, st);
         if (o.ok) {
             acc[0] += g.sun.x;
             acc[1] += g.sun.y;
@@ -414,31 +540,16 @@ __global__ void __launch_bounds__(32 * ROWS, LH_BWD_MIN_BLOCKS * 8 / ROWS)
         }
         if (tex_targets) {
             // base colour (rgb of the texel) and metallic-roughness (g, b)
-            float* ba[4] = {nullptr, nullptr, nullptr, nullptr};
-            float* ma[4] = {nullptr, nullptr, nullptr, nullptr};
-            bool base_small = false, mr_small = false;
-            if (o.ok && g.base_index < f.n_textures && tex_targets[g.base_index]) {
-                const lh_texture& tx = f.textures[g.base_index];
-                float4* dst = reinterpret_cast<float4*>(tex_targets[g.base_index]);
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    ba[q] = reinterpret_cast<float*>(dst + (size_t)g.base_ij[2 + (q >> 1)] * tx.width + g.base_ij[q & 1]);
-                base_small = tx.width * tx.height <= kSmallTexture;
-            }
-            if (o.ok && g.mr_index < f.n_textures && tex_targets[g.mr_index]) {
-                const lh_texture& tx = f.textures[g.mr_index];
-                float4* dst = reinterpret_cast<float4*>(tex_targets[g.mr_index]);
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    ma[q] = reinterpret_cast<float*>(dst + (size_t)g.mr_ij[2 + (q >> 1)] * tx.width + g.mr_ij[q & 1]);
-                mr_small = tx.width * tx.height <= kSmallTexture;
-            }
-            scatter_texels<3>(cache, ba, g.base_texel, 0, base_small);
-            scatter_texels<2>(cache, ma, g.mr_texel, 1, mr_small);  // roughness (g), metallic (b)
+            const uint32_t bi = o.ok && g.base_index < f.n_textures ? g.base_index : 0u;
+            const uint32_t mi = o.ok && g.mr_index < f.n_textures ? g.mr_index : 0u;
+            float* base = o.ok && g.base_index < f.n_textures ? reinterpret_cast<float*>(tex_targets[bi]) : nullptr;
+            float* mr = o.ok && g.mr_index < f.n_textures ? reinterpret_cast<float*>(tex_targets[mi]) : nullptr;
+            scatter_texels<3>(cache, base, f.textures[bi], g.base_ij, g.base_texel, 0);
+            scatter_texels<2>(cache, mr, f.textures[mi], g.mr_ij, g.mr_texel, 1);  // roughness (g), metallic (b)
         }
         // the geometry half of the reverse, then the vertex attributes: one
         // run per triangle
-        if (o.ok) shade::shade_geometry<float>(fx, p, st, &g);
+        if (o.ok) shade::shade_geometry<float>(fx, tri, st, &g);
         if (__any_sync(kFull, mg != nullptr)) {
             const Run r = run_of(mg ? (unsigned long long)o.packed : ~0ull);
             float v[24];
@@ -464,18 +575,12 @@ __global__ void __launch_bounds__(32 * ROWS, LH_BWD_MIN_BLOCKS * 8 / ROWS)
                     const float* vk = v + k * 8;
                     if (d.positions) {
                         // W = M3 P + t: dP = M3^T dW
-                        float* p = reinterpret_cast<float*>(d.positions) + (size_t)o.idx[k] * 3;
                         const f3 gw{vk[0], vk[1], vk[2]};
-                        atomicAdd(p, dot(c0, gw));
-                        atomicAdd(p + 1, dot(c1, gw));
-                        atomicAdd(p + 2, dot(c2, gw));
+                        add3(reinterpret_cast<float*>(d.positions) + (size_t)o.idx[k] * 3,
+                             f3{dot(c0, gw), dot(c1, gw), dot(c2, gw)});
                     }
-                    if (d.normals) {
-                        float* p = reinterpret_cast<float*>(d.normals) + (size_t)o.idx[k] * 3;
-                        atomicAdd(p, vk[3]);
-                        atomicAdd(p + 1, vk[4]);
-                        atomicAdd(p + 2, vk[5]);
-                    }
+                    if (d.normals)
+                        add3(reinterpret_cast<float*>(d.normals) + (size_t)o.idx[k] * 3, f3{vk[3], vk[4], vk[5]});
                     if (d.uvs) {
                         float* p = reinterpret_cast<float*>(d.uvs) + (size_t)o.idx[k] * 2;
                         if (((uintptr_t)p & 7u) == 0) {
@@ -511,21 +616,24 @@ int g_backward_blocks_per_sm[3] = {-1, -1, -1};
 template <int ROWS>
 cudaError_t launch_backward_rows(const FrameDev& f, uint32_t width, uint32_t height, const float4* grad,
                                  const lh_grad_targets& t, cudaStream_t s, int& blocks_per_sm) {
+    constexpr uint32_t kShared = ROWS * kTerms * 32 * (uint32_t)sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(k_resolve_backward<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShared);
+    if (e != cudaSuccess) return e;
     if (blocks_per_sm < 0) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_resolve_backward<ROWS>, 32 * ROWS, 0) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_resolve_backward<ROWS>, 32 * ROWS, kShared) != cudaSuccess)
             n = 1;
         blocks_per_sm = n > 0 ? n : 1;
     }
     int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     const uint32_t tiles_x = (width + 31) / 32, tiles_y = (height + ROWS - 1) / ROWS;
     const uint32_t n_tiles = tiles_x * tiles_y;
     if (n_tiles == 0) return cudaSuccess;
     const uint32_t grid = std::min<uint32_t>(n_tiles, (uint32_t)(sms * blocks_per_sm));
-    return launch_pdl(k_resolve_backward<ROWS>, dim3(grid), dim3(32, ROWS), s, f, grad, t, tiles_x, n_tiles);
+    return launch_pdl_shared(k_resolve_backward<ROWS>, dim3(grid), dim3(32, ROWS), kShared, s, f, grad, t, tiles_x, n_tiles);
 }
 
 }  // namespace

@@ -180,11 +180,12 @@ struct FrameDev {
 #define LH_PDL 1
 #endif
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+cudaError_t launch_pdl_shared(void (*kernel)(KArgs...), dim3 grid, dim3 block, uint32_t shared, cudaStream_t s,
+                              Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = shared;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -195,6 +196,10 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStre
     if (e != cudaSuccess) return e;
     cfg.numAttrs = LH_PDL && capture == cudaStreamCaptureStatusNone ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+    return launch_pdl_shared(kernel, grid, block, 0u, s, args...);
 }
 
 // Launchers (stream ordered).  Each returns the CUDA error of its launch.

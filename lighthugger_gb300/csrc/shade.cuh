@@ -95,26 +95,16 @@ template <class T> LH_HD T pow4(T x) {
     return x2 * x2;
 }
 template <class T> LH_HD T pow5(T x) { return pow4(x) * x; }
+template <class T> LH_HD T inv_length(v3<T> v) { return fdiv(T(1), fsqrt(dot(v, v))); }
 template <class T> LH_HD v3<T> fnormalize(v3<T> v) {
-    const T r = fdiv(T(1), fsqrt(dot(v, v)));
+    const T r = inv_length(v);
     return {v.x * r, v.y * r, v.z * r};
 }
 // reverse of y = normalize(x): gx = (gy - y (y . gy)) / |x|
-template <class T> LH_HD v3<T> fnormalize_adj(v3<T> x, v3<T> y, v3<T> gy) {
-    const T r = fdiv(T(1), fsqrt(dot(x, x)));
+// (r = 1 / |x|)
+template <class T> LH_HD v3<T> fnormalize_adj(T r, v3<T> y, v3<T> gy) {
     const T d = dot(y, gy);
     return {(gy.x - y.x * d) * r, (gy.y - y.y * d) * r, (gy.z - y.z * d) * r};
-}
-
-// Keeps the device compiler from merging a recomputation with the first
-// computation of the same values (a no-op on the host).
-LH_HD void opaque(double&) {}
-LH_HD void opaque(float& x) {
-#if defined(__CUDA_ARCH__)
-    asm volatile("" : "+f"(x));
-#else
-    (void)x;
-#endif
 }
 
 // One bilinear sample: the 4 texels (linear values) and the weights' inputs.
@@ -226,6 +216,8 @@ template <class T> struct PixelGrad {
     bool differentiated;
 };
 
+constexpr uint64_t kAllPass = (1ull << 36) - 1;  // every compare of the 9 taps passed
+
 // Compare results of one PCF tap (4 bits: texels 00, 10, 01, 11); the
 // sampler's shadow_cmp(layer, i, j, ref) is 1 when ref < stored.
 template <class T, class Sampler>
@@ -281,43 +273,77 @@ template <class T> LH_HD BurleyOut<T> burley(T NoV, T NoL, T LoH, T a) {
 
 // The world position the forward interpolates (CalcFullBary's lambda and
 // InterpolateWithDeriv), in the IEEE arithmetic of the inputs given: it
-// selects the cascade and places the PCF taps.
+// selects the cascade and places the PCF taps.  First the triangle's own
+// terms, then a pixel's.
+template <class T> struct WorldTerms {
+    v2<T> n0;
+    T iw0;
+    T ddx[3], ddy[3];
+    T sx, sy;
+};
+// A triangle's projected vertices `n` and `iw` = 1 / w: vertex k's part of
+// the screen derivatives of lambda / w (inv_det = 1 / bary_det(n)).
+template <class T> LH_HD T bary_det(v2<T> n0, v2<T> n1, v2<T> n2) {
+    v2<T> ca{n2.x - n1.x, n2.y - n1.y}, cb{n0.x - n1.x, n0.y - n1.y};
+    return ca.x * cb.y - cb.x * ca.y;
+}
+template <class T> LH_HD v2<T> bary_slope(v2<T> next, v2<T> after, T inv_det, T iw) {
+    return {(next.y - after.y) * inv_det * iw, (after.x - next.x) * inv_det * iw};
+}
+template <class T> LH_HD T sum_slopes(T a, T b, T c) { return (a * T(1) + b * T(1)) + c * T(1); }
+
+template <class T, class Tri>
+LH_HD v3<T> world_at(const Tri& tri, T ndc_x, T ndc_y) {
+    const WorldTerms<T> w = tri.world_terms();
+    v2<T> dv{ndc_x - w.n0.x, ndc_y - w.n0.y};
+    T wi = T(1) / ((w.iw0 + dv.x * w.sx) + dv.y * w.sy);
+    T lam[3] = {wi * ((w.iw0 + dv.x * w.ddx[0]) + dv.y * w.ddy[0]), wi * ((T(0) + dv.x * w.ddx[1]) + dv.y * w.ddy[1]),
+                wi * ((T(0) + dv.x * w.ddx[2]) + dv.y * w.ddy[2])};
+    const v3<T> a = tri.W(0), b = tri.W(1), c = tri.W(2);
+    return {(a.x * lam[0] + b.x * lam[1]) + c.x * lam[2], (a.y * lam[0] + b.y * lam[1]) + c.y * lam[2],
+            (a.z * lam[0] + b.z * lam[1]) + c.z * lam[2]};
+}
+
 template <class T, class F> LH_HD v3<T> forward_world(const F& fx, const PixelParams<T>& p) {
-    v3<T> C[3];
+    struct {
+        WorldTerms<T> w;
+        v3<T> v[3];
+        LH_HD WorldTerms<T> world_terms() const { return w; }
+        LH_HD v3<T> W(int k) const { return v[k]; }
+    } tri;
     T iw[3];
     v2<T> n[3];
     for (int k = 0; k < 3; k++) {
-        C[k] = xform_pv(fx, p.W[k], T(1));
+        tri.v[k] = p.W[k];
+        const v3<T> C = xform_pv(fx, p.W[k], T(1));
         iw[k] = T(1) / xform_pv_w(fx, p.W[k], T(1));
-        n[k] = {C[k].x * iw[k], C[k].y * iw[k]};
+        n[k] = {C.x * iw[k], C.y * iw[k]};
     }
-    v2<T> ca{n[2].x - n[1].x, n[2].y - n[1].y}, cb{n[0].x - n[1].x, n[0].y - n[1].y};
-    T invDet = T(1) / (ca.x * cb.y - cb.x * ca.y);
-    T dxr[3] = {n[1].y - n[2].y, n[2].y - n[0].y, n[0].y - n[1].y};
-    T dyr[3] = {n[2].x - n[1].x, n[0].x - n[2].x, n[1].x - n[0].x};
-    T ddx0[3], ddy0[3];
+    const T inv_det = T(1) / bary_det(n[0], n[1], n[2]);
     for (int k = 0; k < 3; k++) {
-        ddx0[k] = dxr[k] * invDet * iw[k];
-        ddy0[k] = dyr[k] * invDet * iw[k];
+        const v2<T> d = bary_slope(n[(k + 1) % 3], n[(k + 2) % 3], inv_det, iw[k]);
+        tri.w.ddx[k] = d.x;
+        tri.w.ddy[k] = d.y;
     }
-    T sx = (ddx0[0] * T(1) + ddx0[1] * T(1)) + ddx0[2] * T(1);
-    T sy = (ddy0[0] * T(1) + ddy0[1] * T(1)) + ddy0[2] * T(1);
-    v2<T> dv{T(fx.ndc[0]) - n[0].x, T(fx.ndc[1]) - n[0].y};
-    T wi = T(1) / ((iw[0] + dv.x * sx) + dv.y * sy);
-    T lam[3] = {wi * ((iw[0] + dv.x * ddx0[0]) + dv.y * ddy0[0]), wi * ((T(0) + dv.x * ddx0[1]) + dv.y * ddy0[1]),
-                wi * ((T(0) + dv.x * ddx0[2]) + dv.y * ddy0[2])};
-    return {(p.W[0].x * lam[0] + p.W[1].x * lam[1]) + p.W[2].x * lam[2],
-            (p.W[0].y * lam[0] + p.W[1].y * lam[1]) + p.W[2].y * lam[2],
-            (p.W[0].z * lam[0] + p.W[1].z * lam[1]) + p.W[2].z * lam[2]};
+    tri.w.n0 = n[0];
+    tri.w.iw0 = iw[0];
+    tri.w.sx = sum_slopes(tri.w.ddx[0], tri.w.ddx[1], tri.w.ddx[2]);
+    tri.w.sy = sum_slopes(tri.w.ddy[0], tri.w.ddy[1], tri.w.ddy[2]);
+    return world_at(tri, T(fx.ndc[0]), T(fx.ndc[1]));
 }
 
-// The forward's discrete decisions at its world position (face flip,
-// far-plane test, the 36 compare results of fx.cascade's layer).
-template <class T, class F, class Sampler>
-LH_HD void decide_at(F& fx, const PixelParams<T>& p, v3<T> world, const Sampler& smp) {
-    v3<T> V = normalize(sub(v3<T>{T(fx.cam[0]), T(fx.cam[1]), T(fx.cam[2])}, world));
-    v3<T> gn = cross(sub(p.W[1], p.W[0]), sub(p.W[2], p.W[0]));
-    fx.flip = dot(gn, V) < T(0) ? -1.0f : 1.0f;
+// Compare results of the 4 x 4 texels at (i, j): bit 4 * row + column.
+template <class T, class Sampler>
+LH_HD uint32_t compare_window(const Sampler& smp, uint32_t layer, int32_t i, int32_t j, T ref) {
+    uint32_t win = 0;
+    for (int r = 0; r < 4; r++)
+        for (int c = 0; c < 4; c++) win |= (smp.shadow_cmp(layer, i + c, j + r, ref) != T(0) ? 1u : 0u) << (4 * r + c);
+    return win;
+}
+
+// The forward's decisions on the shadow at its world position: the far-plane
+// test and the 36 compare results of fx.cascade's layer.
+template <class T, class F, class Sampler> LH_HD void decide_shadow(F& fx, v3<T> world, const Sampler& smp) {
     v3<T> sc = xform_uvs(fx, world, T(1));
     T scw = xform_uvs_w(fx, world, T(1));
     if (scw != T(1)) sc = {sc.x / scw, sc.y / scw, sc.z / scw};  // x / 1 = x
@@ -336,10 +362,11 @@ LH_HD void decide_at(F& fx, const PixelParams<T>& p, v3<T> world, const Sampler&
         iy[k] = (int32_t)tfloor(vv);
     }
     if (ix[1] == ix[0] + 1 && ix[2] == ix[1] + 1 && iy[1] == iy[0] + 1 && iy[2] == iy[1] + 1) {
-        uint32_t win = 0;  // bit 4 * row + column of the window at (ix[0], iy[0])
-        for (int r = 0; r < 4; r++)
-            for (int c = 0; c < 4; c++)
-                win |= (smp.shadow_cmp(layer, ix[0] + c, iy[0] + r, ref) != T(0) ? 1u : 0u) << (4 * r + c);
+        const uint32_t win = compare_window(smp, layer, ix[0], iy[0], ref);
+        if (win == 0u || win == 0xFFFFu) {  // all taps alike
+            fx.cmp = win ? kAllPass : 0ull;
+            return;
+        }
         uint64_t bits = 0;
         for (int ox = 0; ox < 3; ox++)
             for (int oy = 0; oy < 3; oy++) {
@@ -360,21 +387,72 @@ LH_HD void decide_at(F& fx, const PixelParams<T>& p, v3<T> world, const Sampler&
     fx.cmp = bits;
 }
 
+// The face flip as well, from the vertices.
+template <class T, class F, class Sampler>
+LH_HD void decide_at(F& fx, const PixelParams<T>& p, v3<T> world, const Sampler& smp) {
+    v3<T> V = normalize(sub(v3<T>{T(fx.cam[0]), T(fx.cam[1]), T(fx.cam[2])}, world));
+    v3<T> gn = cross(sub(p.W[1], p.W[0]), sub(p.W[2], p.W[0]));
+    fx.flip = dot(gn, V) < T(0) ? -1.0f : 1.0f;
+    decide_shadow(fx, world, smp);
+}
+
 template <class T, class F, class Sampler> LH_HD void decide(F& fx, const PixelParams<T>& p, const Sampler& smp) {
     decide_at(fx, p, forward_world(fx, p), smp);
 }
 
-// Forward geometry of a pixel in two parts: CalcFullBary's lambda and its
-// intermediates (the screen derivatives only feed the normal map, which is
-// not differentiated), then the interpolated world position / uv / normal
-// and the view vector.
+// The terms of a triangle that all its pixels share, in the arithmetic of the
+// continuous part: positions, normalised normals with the reciprocal of their
+// lengths, scaled uvs, clip-space x and y, projected vertices, and
+// CalcFullBary's slopes.  Read through the accessors, so that the device can
+// keep them in shared memory.
+template <class T> struct TriTerms {
+    v3<T> w_[3], nk_[3];
+    T rn_[3], iw_[3], inv_det_;
+    v2<T> uvs_[3], c_[3], n_[3], dd_[3], s_, ts_, toff_;
+    LH_HD v3<T> W(int k) const { return w_[k]; }        // position
+    LH_HD v3<T> nk(int k) const { return nk_[k]; }      // normal, normalised
+    LH_HD T rn(int k) const { return rn_[k]; }          // 1 / |raw normal|
+    LH_HD v2<T> uvs(int k) const { return uvs_[k]; }    // uv times the texture scale
+    LH_HD v2<T> C(int k) const { return c_[k]; }        // clip x, y
+    LH_HD T iw(int k) const { return iw_[k]; }          // 1 / clip w
+    LH_HD v2<T> n(int k) const { return n_[k]; }        // projected x, y
+    LH_HD v2<T> dd(int k) const { return dd_[k]; }      // slopes of lambda_k / w in x and y
+    LH_HD v2<T> s() const { return s_; }                // their sums
+    LH_HD T inv_det() const { return inv_det_; }
+    LH_HD v2<T> ts() const { return ts_; }              // texture scale and offset
+    LH_HD v2<T> toff() const { return toff_; }
+};
+
+// A vertex's projection: clip x, y and 1 / w.
+template <class T, class F> LH_HD T project(const F& fx, v3<T> W, v2<T>& c, v2<T>& n) {
+    const v3<T> C = xform_pv(fx, W, T(1));
+    const T iw = fdiv(T(1), xform_pv_w(fx, W, T(1)));
+    c = {C.x, C.y};
+    n = {C.x * iw, C.y * iw};
+    return iw;
+}
+
+template <class T, class F> LH_HD TriTerms<T> tri_terms(const F& fx, const PixelParams<T>& p) {
+    TriTerms<T> t;
+    for (int k = 0; k < 3; k++) {
+        t.w_[k] = p.W[k];
+        t.rn_[k] = inv_length(p.N[k]);
+        t.nk_[k] = mul(p.N[k], t.rn_[k]);
+        t.uvs_[k] = {p.UV[k].x * T(fx.ts[0]), p.UV[k].y * T(fx.ts[1])};
+        t.iw_[k] = project(fx, p.W[k], t.c_[k], t.n_[k]);
+    }
+    t.inv_det_ = fdiv(T(1), bary_det(t.n_[0], t.n_[1], t.n_[2]));
+    for (int k = 0; k < 3; k++) t.dd_[k] = bary_slope(t.n_[(k + 1) % 3], t.n_[(k + 2) % 3], t.inv_det_, t.iw_[k]);
+    t.s_ = {sum_slopes(t.dd_[0].x, t.dd_[1].x, t.dd_[2].x), sum_slopes(t.dd_[0].y, t.dd_[1].y, t.dd_[2].y)};
+    t.ts_ = {T(fx.ts[0]), T(fx.ts[1])};
+    t.toff_ = {T(fx.toff[0]), T(fx.toff[1])};
+    return t;
+}
+
+// Forward geometry of a pixel in two parts: CalcFullBary's lambda (the screen
+// derivatives only feed the normal map, which is not differentiated), then
+// the interpolated world position / uv / normal and the view vector.
 template <class T> struct Bary {
-    v3<T> C[3];
-    T iw[3];
-    v2<T> ca, cb;
-    T invDet;
-    T dxr[3], dyr[3], ddx0[3], ddy0[3];
-    T sx, sy;
     v2<T> dv;
     T wi;
     T av[3], lam[3];
@@ -388,49 +466,31 @@ template <class T> struct Interp {
     v3<T> nt, n0, normal;
 };
 
-template <class T, class F> LH_HD void bary(const F& fx, const PixelParams<T>& p, Bary<T>& B) {
-    v2<T> n[3];
+template <class T, class F, class Tri> LH_HD void bary(const F& fx, const Tri& tri, Bary<T>& B) {
+    const v2<T> n0 = tri.n(0), s = tri.s();
+    const T iw0 = tri.iw(0);
+    B.dv = {T(fx.ndc[0]) - n0.x, T(fx.ndc[1]) - n0.y};
+    B.wi = fdiv(T(1), (iw0 + B.dv.x * s.x) + B.dv.y * s.y);
     for (int k = 0; k < 3; k++) {
-        B.C[k] = xform_pv(fx, p.W[k], T(1));
-        B.iw[k] = fdiv(T(1), xform_pv_w(fx, p.W[k], T(1)));
-        n[k] = {B.C[k].x * B.iw[k], B.C[k].y * B.iw[k]};
+        const v2<T> d = tri.dd(k);
+        B.av[k] = ((k == 0 ? iw0 : T(0)) + B.dv.x * d.x) + B.dv.y * d.y;
+        B.lam[k] = B.wi * B.av[k];
     }
-    B.ca = {n[2].x - n[1].x, n[2].y - n[1].y};
-    B.cb = {n[0].x - n[1].x, n[0].y - n[1].y};
-    B.invDet = fdiv(T(1), B.ca.x * B.cb.y - B.cb.x * B.ca.y);
-    B.dxr[0] = n[1].y - n[2].y;
-    B.dxr[1] = n[2].y - n[0].y;
-    B.dxr[2] = n[0].y - n[1].y;
-    B.dyr[0] = n[2].x - n[1].x;
-    B.dyr[1] = n[0].x - n[2].x;
-    B.dyr[2] = n[1].x - n[0].x;
-    for (int k = 0; k < 3; k++) {
-        B.ddx0[k] = B.dxr[k] * B.invDet * B.iw[k];
-        B.ddy0[k] = B.dyr[k] * B.invDet * B.iw[k];
-    }
-    B.sx = (B.ddx0[0] * T(1) + B.ddx0[1] * T(1)) + B.ddx0[2] * T(1);
-    B.sy = (B.ddy0[0] * T(1) + B.ddy0[1] * T(1)) + B.ddy0[2] * T(1);
-    B.dv = {T(fx.ndc[0]) - n[0].x, T(fx.ndc[1]) - n[0].y};
-    B.wi = fdiv(T(1), (B.iw[0] + B.dv.x * B.sx) + B.dv.y * B.sy);
-    B.av[0] = (B.iw[0] + B.dv.x * B.ddx0[0]) + B.dv.y * B.ddy0[0];
-    B.av[1] = (T(0) + B.dv.x * B.ddx0[1]) + B.dv.y * B.ddy0[1];
-    B.av[2] = (T(0) + B.dv.x * B.ddx0[2]) + B.dv.y * B.ddy0[2];
-    for (int k = 0; k < 3; k++) B.lam[k] = B.wi * B.av[k];
 }
 
-template <class T, class F>
-LH_HD void interp(const F& fx, const PixelParams<T>& p, const T lam[3], Interp<T>& I) {
+template <class T, class F, class Tri>
+LH_HD void interp(const F& fx, const Tri& tri, const T lam[3], Interp<T>& I) {
     // InterpolateWithDeriv value: dot(v, lambda)
-    I.world = {(p.W[0].x * lam[0] + p.W[1].x * lam[1]) + p.W[2].x * lam[2],
-               (p.W[0].y * lam[0] + p.W[1].y * lam[1]) + p.W[2].y * lam[2],
-               (p.W[0].z * lam[0] + p.W[1].z * lam[1]) + p.W[2].z * lam[2]};
-    v2<T> uvs[3];
-    for (int k = 0; k < 3; k++) uvs[k] = {p.UV[k].x * T(fx.ts[0]), p.UV[k].y * T(fx.ts[1])};
-    I.uv = {((uvs[0].x * lam[0] + uvs[1].x * lam[1]) + uvs[2].x * lam[2]) + T(fx.toff[0]),
-            ((uvs[0].y * lam[0] + uvs[1].y * lam[1]) + uvs[2].y * lam[2]) + T(fx.toff[1])};
+    const v3<T> W[3] = {tri.W(0), tri.W(1), tri.W(2)};
+    I.world = {(W[0].x * lam[0] + W[1].x * lam[1]) + W[2].x * lam[2],
+               (W[0].y * lam[0] + W[1].y * lam[1]) + W[2].y * lam[2],
+               (W[0].z * lam[0] + W[1].z * lam[1]) + W[2].z * lam[2]};
+    const v2<T> uvs[3] = {tri.uvs(0), tri.uvs(1), tri.uvs(2)}, toff = tri.toff();
+    I.uv = {((uvs[0].x * lam[0] + uvs[1].x * lam[1]) + uvs[2].x * lam[2]) + toff.x,
+            ((uvs[0].y * lam[0] + uvs[1].y * lam[1]) + uvs[2].y * lam[2]) + toff.y};
     I.vd = sub(v3<T>{T(fx.cam[0]), T(fx.cam[1]), T(fx.cam[2])}, I.world);
     I.V = fnormalize(I.vd);
-    for (int k = 0; k < 3; k++) I.nk[k] = fnormalize(p.N[k]);
+    for (int k = 0; k < 3; k++) I.nk[k] = tri.nk(k);
     const v3<T> ni = {(I.nk[0].x * lam[0] + I.nk[1].x * lam[1]) + I.nk[2].x * lam[2],
                       (I.nk[0].y * lam[0] + I.nk[1].y * lam[1]) + I.nk[2].y * lam[2],
                       (I.nk[0].z * lam[0] + I.nk[1].z * lam[1]) + I.nk[2].z * lam[2]};
@@ -454,8 +514,23 @@ template <class T, class F> LH_HD ShadowTerm<T> shadow_term(const F& fx, v3<T> w
     sc = {sc.x * inv_w, sc.y * inv_w, sc.z * inv_w};
     T shadow = T(0), dsx = T(0), dsy = T(0);
     const T S = T(fx.shadow_size);
-    // with every compare 0 each tap's value and derivatives are exactly 0
-    if (fx.cmp != 0) {
+    // with every compare 0 each tap's value and derivatives are exactly 0;
+    // with every compare 1 the derivatives are, and the value is the weights'
+    // sum (its rounding included), by a fifth of the arithmetic
+    if (fx.cmp == kAllPass) {
+        T a[3], b[3];
+        for (int k = 0; k < 3; k++) {
+            T uu = (sc.x + T(k - 1) / T(1024)) * S - T(0.5), vv = (sc.y + T(k - 1) / T(1024)) * S - T(0.5);
+            if (!(tabs(uu) < T(1e9))) uu = T(0);
+            if (!(tabs(vv) < T(1e9))) vv = T(0);
+            a[k] = uu - tfloor(uu);
+            b[k] = vv - tfloor(vv);
+        }
+        for (int ox = 0; ox < 3; ox++)
+            for (int oy = 0; oy < 3; oy++)
+                shadow += (((T(1) - a[ox]) * (T(1) - b[oy]) + a[ox] * (T(1) - b[oy])) + (T(1) - a[ox]) * b[oy]) +
+                          a[ox] * b[oy];
+    } else if (fx.cmp != 0) {
         for (int ox = -1; ox <= 1; ox++)
             for (int oy = -1; oy <= 1; oy++) {
                 T da, db;
@@ -628,7 +703,7 @@ LH_HD void surface(const F& fx, const PixelParams<T>& p, const Sampler& smp, v2<
     g_V = add(g_V, mul(normal, g_NoV));
     g_L = add(g_L, add(mul(normal, g_NoL), mul(H, g_LoH)));
     v3<T> g_H = add(mul(normal, g_NoH), mul(L, g_LoH));
-    v3<T> g_h0 = fnormalize_adj(h0, H, g_H);
+    v3<T> g_h0 = fnormalize_adj(inv_length(h0), H, g_H);
     g_V = add(g_V, g_h0);
     g_L = add(g_L, g_h0);
     g->sun = g_L;
@@ -671,65 +746,47 @@ LH_HD void surface(const F& fx, const PixelParams<T>& p, const Sampler& smp, v2<
     sg->uv = g_uv;
 }
 
-// Opaque copies of the vertex attributes: a recomputation from them is not
-// merged with an earlier one by the device compiler.
-template <class T> LH_HD PixelParams<T> opaque_params(PixelParams<T> p) {
-    for (int k = 0; k < 3; k++) {
-        opaque(p.W[k].x), opaque(p.W[k].y), opaque(p.W[k].z);
-        opaque(p.N[k].x), opaque(p.N[k].y), opaque(p.N[k].z);
-        opaque(p.UV[k].x), opaque(p.UV[k].y);
-    }
-    return p;
-}
-
 // Reverse of the geometry: from the gradients of the surface inputs (and of
 // the world position through the shadow term) to the vertex attributes.
-// The forward geometry is recomputed here in two steps -- the lambdas and
-// interpolants for the first half of the reverse, the barycentric
-// intermediates again for the second -- so that only a few values are live
-// at any point.
-template <class T, class F>
-LH_HD void geometry_adjoint(const F& fx, const PixelParams<T>& p0, const SurfaceGrad<T>& sg, v3<T> g_world,
-                            PixelGrad<T>* g) {
-    T lam[3], g_lam[3];
+// The forward geometry is recomputed here rather than kept, so that only a
+// few values are live at any point.
+template <class T, class F, class Tri>
+LH_HD void geometry_adjoint(const F& fx, const Tri& tri, const SurfaceGrad<T>& sg, v3<T> g_world, PixelGrad<T>* g) {
+    Bary<T> G;
+    bary(fx, tri, G);
+    const T* lam = G.lam;
+    T g_lam[3];
     {
-        const PixelParams<T> p = opaque_params(p0);
-        {
-            Bary<T> B;
-            bary(fx, p, B);
-            lam[0] = B.lam[0];
-            lam[1] = B.lam[1];
-            lam[2] = B.lam[2];
-        }
         Interp<T> I;
-        interp(fx, p, lam, I);
+        interp(fx, tri, lam, I);
         // normal = flip * normalize(nt); nt = NT ni; ni = sum lam_k nk; nk = normalize(N_k)
         v3<T> g_n0 = mul(sg.normal, T(fx.flip));
-        v3<T> g_nt = fnormalize_adj(I.nt, I.n0, g_n0);
+        v3<T> g_nt = fnormalize_adj(inv_length(I.nt), I.n0, g_n0);
         v3<T> g_ni{(T(fx.NT(0, 0)) * g_nt.x + T(fx.NT(0, 1)) * g_nt.y) + T(fx.NT(0, 2)) * g_nt.z,
                    (T(fx.NT(1, 0)) * g_nt.x + T(fx.NT(1, 1)) * g_nt.y) + T(fx.NT(1, 2)) * g_nt.z,
                    (T(fx.NT(2, 0)) * g_nt.x + T(fx.NT(2, 1)) * g_nt.y) + T(fx.NT(2, 2)) * g_nt.z};
         for (int k = 0; k < 3; k++) {
-            g->N[k] = fnormalize_adj(p.N[k], I.nk[k], mul(g_ni, lam[k]));
+            g->N[k] = fnormalize_adj(tri.rn(k), I.nk[k], mul(g_ni, lam[k]));
             g_lam[k] = dot(I.nk[k], g_ni);
         }
         // V = normalize(cam - world)
-        g_world = sub(g_world, fnormalize_adj(I.vd, I.V, sg.V));
+        g_world = sub(g_world, fnormalize_adj(inv_length(I.vd), I.V, sg.V));
         // uv = sum lam_k uvs_k + offset, uvs_k = UV_k * scale
+        const v2<T> ts = tri.ts();
         for (int k = 0; k < 3; k++) {
-            g->UV[k] = {sg.uv.x * lam[k] * T(fx.ts[0]), sg.uv.y * lam[k] * T(fx.ts[1])};
-            g_lam[k] += sg.uv.x * (p.UV[k].x * T(fx.ts[0])) + sg.uv.y * (p.UV[k].y * T(fx.ts[1]));
+            const v2<T> uvs = tri.uvs(k);
+            g->UV[k] = {sg.uv.x * lam[k] * ts.x, sg.uv.y * lam[k] * ts.y};
+            g_lam[k] += sg.uv.x * uvs.x + sg.uv.y * uvs.y;
         }
         // world = sum lam_k W_k.  The lambdas sum to 1 for every input, so
         // their gradients may be shifted by a common term: W_k - W_0 instead
         // of W_k keeps float32 from cancelling world-scale coordinates.
+        const v3<T> W0 = tri.W(0);
         for (int k = 0; k < 3; k++) {
             g->W[k] = mul(g_world, lam[k]);
-            g_lam[k] += dot(sub(p.W[k], p.W[0]), g_world);
+            g_lam[k] += dot(sub(tri.W(k), W0), g_world);
         }
     }
-    Bary<T> G;
-    bary(fx, opaque_params(p0), G);
     // ---- barycentrics: lam_k = wi * av_k
     const T wi = G.wi;
     T g_wi = (g_lam[0] * G.av[0] + g_lam[1] * G.av[1]) + g_lam[2] * G.av[2];
@@ -739,26 +796,32 @@ LH_HD void geometry_adjoint(const F& fx, const PixelParams<T>& p0, const Surface
     T g_ddx0[3] = {T(0), T(0), T(0)}, g_ddy0[3] = {T(0), T(0), T(0)};
     v2<T> g_dv{T(0), T(0)};
     g_iw[0] += g_iiw;
-    g_dv.x += g_iiw * G.sx;
-    g_dv.y += g_iiw * G.sy;
+    const v2<T> s = tri.s();
+    g_dv.x += g_iiw * s.x;
+    g_dv.y += g_iiw * s.y;
     T g_sx = g_iiw * G.dv.x, g_sy = g_iiw * G.dv.y;
     g_iw[0] += g_av[0];
     for (int k = 0; k < 3; k++) {
-        g_dv.x += g_av[k] * G.ddx0[k];
-        g_dv.y += g_av[k] * G.ddy0[k];
+        const v2<T> d = tri.dd(k);
+        g_dv.x += g_av[k] * d.x;
+        g_dv.y += g_av[k] * d.y;
         g_ddx0[k] += g_av[k] * G.dv.x + g_sx;
         g_ddy0[k] += g_av[k] * G.dv.y + g_sy;
     }
+    const v2<T> n[3] = {tri.n(0), tri.n(1), tri.n(2)};
+    const T iw[3] = {tri.iw(0), tri.iw(1), tri.iw(2)}, invDet = tri.inv_det();
+    const v2<T> ca{n[2].x - n[1].x, n[2].y - n[1].y}, cb{n[0].x - n[1].x, n[0].y - n[1].y};
     T g_invDet = T(0), g_dxr[3], g_dyr[3];
     for (int k = 0; k < 3; k++) {
-        g_dxr[k] = g_ddx0[k] * G.invDet * G.iw[k];
-        g_dyr[k] = g_ddy0[k] * G.invDet * G.iw[k];
-        g_invDet += g_ddx0[k] * G.dxr[k] * G.iw[k] + g_ddy0[k] * G.dyr[k] * G.iw[k];
-        g_iw[k] += g_ddx0[k] * G.dxr[k] * G.invDet + g_ddy0[k] * G.dyr[k] * G.invDet;
+        const T dxr = n[(k + 1) % 3].y - n[(k + 2) % 3].y, dyr = n[(k + 2) % 3].x - n[(k + 1) % 3].x;
+        g_dxr[k] = g_ddx0[k] * invDet * iw[k];
+        g_dyr[k] = g_ddy0[k] * invDet * iw[k];
+        g_invDet += g_ddx0[k] * dxr * iw[k] + g_ddy0[k] * dyr * iw[k];
+        g_iw[k] += g_ddx0[k] * dxr * invDet + g_ddy0[k] * dyr * invDet;
     }
     v2<T> g_n[3] = {{-g_dv.x, -g_dv.y}, {T(0), T(0)}, {T(0), T(0)}};
-    T g_det = -g_invDet * G.invDet * G.invDet;
-    v2<T> g_ca{g_det * G.cb.y, -g_det * G.cb.x}, g_cb{-g_det * G.ca.y, g_det * G.ca.x};
+    T g_det = -g_invDet * invDet * invDet;
+    v2<T> g_ca{g_det * cb.y, -g_det * cb.x}, g_cb{-g_det * ca.y, g_det * ca.x};
     g_n[2].x += g_ca.x; g_n[2].y += g_ca.y; g_n[1].x -= g_ca.x; g_n[1].y -= g_ca.y;
     g_n[0].x += g_cb.x; g_n[0].y += g_cb.y; g_n[1].x -= g_cb.x; g_n[1].y -= g_cb.y;
     g_n[1].y += g_dxr[0] - g_dxr[2];
@@ -769,9 +832,10 @@ LH_HD void geometry_adjoint(const F& fx, const PixelParams<T>& p0, const Surface
     g_n[0].x += g_dyr[1] - g_dyr[2];
     for (int k = 0; k < 3; k++) {
         // n_k = C_k.xy * iw_k, iw_k = 1 / C_k.w
-        T gCx = g_n[k].x * G.iw[k], gCy = g_n[k].y * G.iw[k];
-        g_iw[k] += g_n[k].x * G.C[k].x + g_n[k].y * G.C[k].y;
-        T gCw = -g_iw[k] * G.iw[k] * G.iw[k];
+        const v2<T> C = tri.C(k);
+        T gCx = g_n[k].x * iw[k], gCy = g_n[k].y * iw[k];
+        g_iw[k] += g_n[k].x * C.x + g_n[k].y * C.y;
+        T gCw = -g_iw[k] * iw[k] * iw[k];
         // C = PV (W, 1): dW_j = sum_r PV[j][r] dC_r  (C.z carries no gradient)
         g->W[k].x += (T(fx.PV(0, 0)) * gCx + T(fx.PV(0, 1)) * gCy) + T(fx.PV(0, 3)) * gCw;
         g->W[k].y += (T(fx.PV(1, 0)) * gCx + T(fx.PV(1, 1)) * gCy) + T(fx.PV(1, 3)) * gCw;
@@ -788,20 +852,20 @@ template <class T> struct SurfaceState {
     SurfaceGrad<T> sg;
 };
 
-template <class T, class F, class Sampler>
-LH_HD void shade_surface(const F& fx, const PixelParams<T>& p, const Sampler& smp, v3<T>* out, v3<T> gout,
-                         PixelGrad<T>* g, SurfaceState<T>* st) {
+template <class T, class F, class Tri, class Sampler>
+LH_HD void shade_surface(const F& fx, const PixelParams<T>& p, const Tri& tri, const Sampler& smp, v3<T>* out,
+                         v3<T> gout, PixelGrad<T>* g, SurfaceState<T>* st) {
     Bary<T> B;
-    bary(fx, p, B);
+    bary(fx, tri, B);
     Interp<T> I;
-    interp(fx, p, B.lam, I);
+    interp(fx, tri, B.lam, I);
     st->sh = shadow_term(fx, I.world);
     surface(fx, p, smp, I.uv, I.normal, I.V, st->sh.value, out, gout, g, &st->sg);
     if (g) g->differentiated = fx.has_normal_map == 0;
 }
 
-template <class T, class F>
-LH_HD void shade_geometry(const F& fx, const PixelParams<T>& p, const SurfaceState<T>& st, PixelGrad<T>* g) {
+template <class T, class F, class Tri>
+LH_HD void shade_geometry(const F& fx, const Tri& tri, const SurfaceState<T>& st, PixelGrad<T>* g) {
     // shadow: d/d(sc.xy) through the PCF weights, compare results fixed;
     // sc.xy = (UVS (world,1)).xy / w with w = row 3 (constant 1 for the
     // orthographic cascades)
@@ -815,7 +879,7 @@ LH_HD void shade_geometry(const F& fx, const PixelParams<T>& p, const SurfaceSta
         g_world.y = (T(fx.UVS(1, 0)) * gsx + T(fx.UVS(1, 1)) * gsy) + T(fx.UVS(1, 3)) * gw;
         g_world.z = (T(fx.UVS(2, 0)) * gsx + T(fx.UVS(2, 1)) * gsy) + T(fx.UVS(2, 3)) * gw;
     }
-    geometry_adjoint(fx, p, st.sg, g_world, g);
+    geometry_adjoint(fx, tri, st.sg, g_world, g);
 }
 
 // Forward (into *out) and, when `g` is non-null, the reverse pass for the
@@ -826,9 +890,10 @@ LH_HD void shade_geometry(const F& fx, const PixelParams<T>& p, const SurfaceSta
 // coordinates.  `smp` provides sample(tex, uv) -> Bilinear.
 template <class T, class F, class Sampler>
 LH_HD void shade(const F& fx, const PixelParams<T>& p, const Sampler& smp, v3<T>* out, v3<T> gout, PixelGrad<T>* g) {
+    const TriTerms<T> tri = tri_terms(fx, p);
     SurfaceState<T> st;
-    shade_surface(fx, p, smp, out, gout, g, &st);
-    if (g) shade_geometry(fx, p, st, g);
+    shade_surface(fx, p, tri, smp, out, gout, g, &st);
+    if (g) shade_geometry(fx, tri, st, g);
 }
 
 }  // namespace shade
