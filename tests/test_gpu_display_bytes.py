@@ -2,7 +2,7 @@
 the sRGB encoding.  The table holds one colour, so each channel is encoded from
 a known value.  Rounding on the way (six blends of a value with itself, a power
 of 2 ulp and the scaling, in float32) moves the code by less than 2e-4, so at
-1e-3 and 3e-3 from a boundary the byte is certain."""
+3e-4 and 3e-3 from a boundary, on both sides of the guard, the byte is certain."""
 import numpy as np
 import pytest
 
@@ -16,7 +16,7 @@ def test_display_bytes_at_the_boundaries(native):
     r = lh.Renderer(lh.Config(width=64, height=36, shadow_size=64, max_instances=1024, max_draws=200000))
     r.set_scene(scene)
     r.frame(scene.uniforms)
-    steps = np.array([-3e-3, -1e-3, 1e-3, 3e-3])
+    steps = np.array([-3e-3, -3e-4, 3e-4, 3e-3])
     code = (np.arange(1, 256)[:, None] + steps[None, :]).reshape(-1)  # before floor, 255 x + 0.5
     encoded = (code - 0.5) / 255.0
     knee = 0.003130 * 12.92
