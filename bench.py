@@ -55,7 +55,8 @@ FRAGMENT_BYTES = 8           # one 64-bit depth-test reduction per fragment
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "dram_bytes_c2_frame.txt")
 # (k_raster_alpha<K> launches only for scenes with alpha-clip meshes)
 STAGE_KERNELS = {
-    "raster": ("k_raster<0>", "k_raster_alpha<0>", "k_raster_big<0>", "k_hiz", "k_occlusion_filter"),
+    "raster": ("k_raster<0>", "k_raster_alpha<0>", "k_raster_big<0>", "k_raster_occluders", "k_hiz",
+               "k_occlusion_filter"),
     "shadow_raster": ("k_raster<1>", "k_raster_alpha<1>", "k_raster_big<1>"),
     "resolve": ("k_resolve<1>",),
     "cull_meshlets": ("k_cull_meshlets",),
@@ -434,7 +435,7 @@ def run_gpu(args):
         # raster the visibility view adds the occluder pass, its chunks, the
         # hierarchical depth and the depth test of the other meshlets; the two
         # alpha-clip launches only when a mesh of the scene is alpha clip
-        "gpu_launches": (13 + (4 if tune.occlusion_px else 0)
+        "gpu_launches": (13 + (4 if tune.occlusion_px and any(st.occlusion) else 0)
                          - (0 if scene.params.get("alpha_clip_materials") else 2)) * args.steps,
         "tuning": dict(tune.as_dict(), autotuned=tune_results),
         "occlusion": {"occluder_px": int(tune.occlusion_px), "occluders": int(st.occlusion[0]),

@@ -268,6 +268,22 @@ size_t reset_bytes_for(const lh_ctx* c) {
     return align_up(kStWords * 4, 256) + per_view * c->max_views;
 }
 
+// The occluder threshold of a frame of n_views views (4 of them cascades).
+// The two-pass raster's four launches cost 14 to 30 us a frame; rasterising
+// what they would have skipped costs about 1 ns a meshlet, so opaque scenes
+// of at most kOnePassMeshlets meshlets, counted once per visibility view, take
+// one pass.  Measured by launches: 3,840 meshlets at 640 x 360 105 -> 91 us,
+// 15,360 at 1280 x 720 116 -> 102, 35,145 (two thirds of the visible ones
+// hidden) 189 -> 161, 44,496 258 -> 232, 145,845 290 -> 262; the other way
+// round 595,594 at 1920 x 1080 336 -> 395 and 498 -> 562, and with
+// alpha-tested meshes, whose hidden pixels cost a texture sample each, 88,261
+// 459 -> 564.  The line lies where no view can gain 30 us.
+constexpr uint64_t kOnePassMeshlets = 32768;
+uint32_t occlusion_px_of(const lh_ctx* c, uint32_t n_views) {
+    const uint64_t visibility_views = n_views > 4 ? n_views - 4 : 1;
+    return !c->scene_alpha && c->scene_meshlets * visibility_views <= kOnePassMeshlets ? 0u : c->tuning.occlusion_px;
+}
+
 FrameDev frame_dev(const lh_ctx* c, uint32_t n_views, uint32_t n_instances) {
     FrameDev f{};
     f.instances = c->instances;
@@ -292,7 +308,7 @@ FrameDev frame_dev(const lh_ctx* c, uint32_t n_views, uint32_t n_instances) {
     f.uniforms = c->d_uniforms;
     f.frame_consts = c->d_consts;
     f.srgb_lut = c->d_srgb;
-    f.occlusion_px = c->tuning.occlusion_px;
+    f.occlusion_px = occlusion_px_of(c, n_views);
     f.scene_alpha = c->scene_alpha ? 1u : 0u;
     for (int k = 0; k < 2; k++) {
         f.chunk_shift[k][0] = (uint32_t)__builtin_ctz(c->tuning.chunk_rows[k]);
@@ -903,7 +919,7 @@ lh_status lh_read_status(lh_ctx* c, lh_device_status* out) {
     out->clipped_triangles = words[kStClipCount];
     out->fragments[0] = words[kStFragVis];
     out->fragments[1] = words[kStFragShadow];
-    if (!c->h_views.empty() && c->tuning.occlusion_px) {
+    if (!c->h_views.empty() && occlusion_px_of(c, c->n_views_last)) {
         uint32_t claim[kClaimWords];
         e = cudaMemcpy(claim, c->h_views[0].claim, sizeof(claim), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_fail(c, e, "status read");
