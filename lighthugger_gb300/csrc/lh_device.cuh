@@ -311,7 +311,7 @@ struct TriSetup {
     uint32_t bias;  // bit0 edge12, bit1 edge20, bit2 edge01 not top-left;
                     // bit3: every edge product in the bbox fits 32 bits;
                     // bit4 (kBiasAlpha): alpha-tested
-    uint32_t verts;  // alpha-tested: meshlet vertices m0 | m1 << 8 | m2 << 16
+    uint32_t verts;  // alpha-tested: meshlet vertices m0 | m1 << 6 | m2 << 12, triangle << 18
 };
 constexpr uint32_t kBiasAlpha = 16u;
 constexpr uint32_t kBiasWhole = 32u;  // BigTri: taken whole by one warp, not by chunks

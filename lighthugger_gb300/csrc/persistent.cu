@@ -82,10 +82,10 @@ __global__ void __launch_bounds__(kPersistentThreads, 3) k_frame_persistent(cons
         phase_occlusion_filter(f, 0, n_persp, gtid, gstride);
         if (!grid_barrier(f, epoch)) return;
         phase_raster<0>(f, 0, n_persp, tune, s_raster.small, kListSurvivors);
-        phase_raster_general<0, true>(f, 0, n_persp, tune, s_raster.alpha, s_raster.alpha.av, kListSurvivors);
+        phase_raster_general<0, true>(f, 0, n_persp, tune, s_raster.alpha, s_raster.alpha.alpha, kListSurvivors);
     } else {
         phase_raster<0>(f, 0, n_persp, tune, s_raster.small, kListAll);
-        phase_raster_general<0, true>(f, 0, n_persp, tune, s_raster.alpha, s_raster.alpha.av, kListAll);
+        phase_raster_general<0, true>(f, 0, n_persp, tune, s_raster.alpha, s_raster.alpha.alpha, kListAll);
     }
     if (!grid_barrier(f, epoch)) return;
     phase_raster_big<0>(f, s_raster.big);
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 3) k_frame_persistent(cons
     phase_cull_meshlets(f, n_persp, 4, &f.status[kStMlClaim]);
     if (!grid_barrier(f, epoch)) return;
     phase_raster<1>(f, n_persp, 4, tune, s_raster.small, kListAll);
-    phase_raster_general<1, true>(f, n_persp, 4, tune, s_raster.alpha, s_raster.alpha.av, kListAll);
+    phase_raster_general<1, true>(f, n_persp, 4, tune, s_raster.alpha, s_raster.alpha.alpha, kListAll);
     if (!grid_barrier(f, epoch)) return;
     phase_raster_big<1>(f, s_raster.big);
 }

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(kRasterWarps * 32, 3)
     k_raster_alpha(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune, uint32_t list) {
     __shared__ RasterSmemAlpha sm;
     pdl_enter();
-    phase_raster_general<KIND, true>(f, view_begin, n_views, tune, sm, sm.av, list);
+    phase_raster_general<KIND, true>(f, view_begin, n_views, tune, sm, sm.alpha, list);
 }
 
 template <int KIND>

@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "edge_run.cuh"
+#include "exact_div.cuh"
 #include "lh_device.cuh"
 #include "lh_internal.cuh"
 
@@ -178,18 +179,36 @@ __device__ __forceinline__ float sample_alpha(const FrameDev& f, uint32_t index,
     const float fu = floorf(u), fv = floorf(v);
     const float a = u - fu, b = v - fv;
     const int32_t i0 = (int32_t)fu, j0 = (int32_t)fv, W = (int32_t)t.width, H = (int32_t)t.height;
-    const int32_t ia = wrap_texel(i0, W), ib = wrap_texel(i0 + 1, W), ja = wrap_texel(j0, H), jb = wrap_texel(j0 + 1, H);
+    // i0 + 1 wraps to the texel after i0's (or 0 past the last)
+    const int32_t ia = wrap_texel(i0, W), ib = ia + 1 == W ? 0 : ia + 1;
+    const int32_t ja = wrap_texel(j0, H), jb = ja + 1 == H ? 0 : ja + 1;
     auto al = [&](int32_t i, int32_t j) { return __ldg(&tex[(size_t)j * W + i].w); };
     const float t00 = al(ia, ja), t10 = al(ib, ja), t01 = al(ia, jb), t11 = al(ib, jb);
     const float w00 = (1.0f - a) * (1.0f - b), w10 = a * (1.0f - b), w01 = (1.0f - a) * b, w11 = a * b;
     return ((t00 * w00 + t10 * w10) + t01 * w01) + t11 * w11;
 }
 
-// True when the fragment at pixel (px, py) of a W x H target survives.
-__device__ __forceinline__ bool alpha_pass(const FrameDev& f, const AlphaTri& t, int32_t px, int32_t py, uint32_t W,
-                                           uint32_t H) {
-    const float nx = (((float)px + 0.5f) / (float)W) * 2.0f - 1.0f;
-    const float ny = (((float)py + 0.5f) / (float)H) * 2.0f - 1.0f;
+// (p + 0.5) / n * 2 - 1 of a pixel column or row: the quotient is that of the
+// integers 2 p + 1 and 2 n, whose reciprocal rcp_2n = 1 / (2 n) gives the same bits.
+__device__ __forceinline__ float pixel_ndc(int32_t p, uint32_t n, float rcp_2n) {
+    const float q = 2 * n <= (uint32_t)kExactDivMaxCount ? div_by_count((float)(2 * p + 1), (float)(2 * n), rcp_2n)
+                                                         : ((float)p + 0.5f) / (float)n;
+    return q * 2.0f - 1.0f;
+}
+
+// A target's size as the alpha test reads it.
+struct AlphaSize {
+    uint32_t W, H;
+    float rcp_2w, rcp_2h;
+};
+__device__ __forceinline__ AlphaSize alpha_size(uint32_t W, uint32_t H) {
+    return {W, H, 1.0f / (float)(2 * W), 1.0f / (float)(2 * H)};
+}
+
+// True when the fragment at pixel (px, py) survives.
+__device__ __forceinline__ bool alpha_pass(const FrameDev& f, const AlphaTri& t, int32_t px, int32_t py, const AlphaSize& s) {
+    const float nx = pixel_ndc(px, s.W, s.rcp_2w);
+    const float ny = pixel_ndc(py, s.H, s.rcp_2h);
     const float e0 = (t.a[0] * nx + t.b[0] * ny) + t.c[0];
     const float e1 = (t.a[1] * nx + t.b[1] * ny) + t.c[1];
     const float e2 = (t.a[2] * nx + t.b[2] * ny) + t.c[2];
@@ -402,18 +421,22 @@ __device__ __noinline__ void clip_triangle(const FrameDev& f, uint32_t view, uin
     }
 }
 
-// Where a warp's alpha-tested triangles find their vertices: the warp's
-// shared AlphaVert array (indexed by TriSetup::verts) and the meshlet's
-// base texture.
+// A warp's covered pixels of alpha-tested triangles, waiting for the test.
+// The test (three divisions and a bilinear sample, over 100 instructions) is
+// taken by 32 covered pixels at a time, of whatever triangles: with the lanes
+// testing their own triangles' pixels 14 of 32 were at work.
+struct AlphaRing {
+    uint32_t tri[64];    // vertices (6 bits each) and triangle of the meshlet
+    uint32_t pixel[64];  // x | y << 16
+    float depth[64];
+};
+// Where the warp's alpha-tested triangles find their vertices: its shared
+// AlphaVert array (indexed by TriSetup::verts) and the meshlet's base texture.
 struct AlphaSrc {
     const AlphaVert* av;
-    uint32_t tex;
-    uint32_t H;
+    uint32_t tex, slot;
+    AlphaSize size;
 };
-
-__device__ __forceinline__ AlphaTri alpha_of(const TriSetup& t, const AlphaSrc& as) {
-    return alpha_setup(as.av[t.verts & 0xFFu], as.av[(t.verts >> 8) & 0xFFu], as.av[(t.verts >> 16) & 0xFFu], as.tex);
-}
 
 // The bbox pixels of one triangle by one lane; `nfrag` counts the fragments
 // written (depth-test reductions issued).
@@ -462,46 +485,19 @@ __device__ __forceinline__ void raster_warp(const TriSetup& t, void* target, uin
     }
 }
 
-// The alpha-tested variants are not inlined: their set-up and sampling
-// state stays out of the register allocation of the opaque paths (the
-// launch bounds cap the whole call tree; alpha triangles are the rare case).
+// The ring's entries [first, first + n), n <= 32: tested and written; returns
+// the lane's fragments.  Not inlined: the set-up and sampling state stays out
+// of the register allocation of the meshlet's loop.
 template <int KIND>
-__device__ __noinline__ uint32_t raster_lane_alpha(const FrameDev& f, const TriSetup& t, void* target, uint32_t W,
-                                                   const AlphaSrc& as) {
-    const AlphaTri at = alpha_of(t, as);
-    uint32_t n = 0;
-    for (int32_t py = t.py0; py <= t.py1; py++)
-        for (int32_t px = t.px0; px <= t.px1; px++) {
-            float d;
-            if (cover(t, px, py, d) && alpha_pass(f, at, px, py, W, as.H)) {
-                write_fragment<KIND>(target, W, px, py, d, t.id);
-                n++;
-            }
-        }
-    return n;
-}
-
-template <int KIND>
-__device__ __noinline__ uint32_t raster_warp_alpha(const FrameDev& f, const TriSetup& t, void* target, uint32_t W,
-                                                   uint32_t lane, const AlphaSrc& as) {
-    const uint32_t w = (uint32_t)(t.px1 - t.px0 + 1);
-    const uint32_t npx = w * (uint32_t)(t.py1 - t.py0 + 1);
-    const float inv_w = 1.0f / (float)w;
-    const AlphaTri at = alpha_of(t, as);
-    uint32_t n = 0;
-    for (uint32_t p = lane; p < npx; p += 32) {
-        int32_t ry = (int32_t)(((float)p + 0.5f) * inv_w);
-        int32_t rx = (int32_t)p - ry * (int32_t)w;
-        if (rx < 0) { ry--; rx += (int32_t)w; }
-        else if (rx >= (int32_t)w) { ry++; rx -= (int32_t)w; }
-        int32_t px = t.px0 + rx, py = t.py0 + ry;
-        float d;
-        if (cover(t, px, py, d) && alpha_pass(f, at, px, py, W, as.H)) {
-            write_fragment<KIND>(target, W, px, py, d, t.id);
-            n++;
-        }
-    }
-    return n;
+__device__ __noinline__ uint32_t alpha_fragments(const FrameDev& f, const AlphaRing& ring, uint32_t first, uint32_t n,
+                                                 const AlphaSrc& as, void* target, uint32_t lane) {
+    if (lane >= n) return 0u;
+    const uint32_t i = (first + lane) & 63u, tri = ring.tri[i], pixel = ring.pixel[i];
+    const int32_t px = (int32_t)(pixel & 0xFFFFu), py = (int32_t)(pixel >> 16);
+    const AlphaTri at = alpha_setup(as.av[tri & 63u], as.av[(tri >> 6) & 63u], as.av[(tri >> 12) & 63u], as.tex);
+    if (!alpha_pass(f, at, px, py, as.size)) return 0u;
+    write_fragment<KIND>(target, as.size.W, px, py, ring.depth[i], LH_PACK_ID(tri >> 18, as.slot));
+    return 1u;
 }
 
 __device__ __forceinline__ TriSetup shfl_setup(const TriSetup& s, int src) {
@@ -515,7 +511,7 @@ __device__ __forceinline__ TriSetup shfl_setup(const TriSetup& s, int src) {
 
 // Shared memory of the raster phase (declared by the calling kernel, so that
 // the persistent kernel's phases reuse one copy).  The alpha-clip class adds
-// an AlphaVert array per warp (RasterSmemAlpha).
+// AlphaVerts and a ring of pixels per warp (RasterSmemAlpha).
 constexpr uint32_t kMicroWords = 4 * 32 * 3 / 4;  // four rounds of 32 triangles (MAX_MESHLET_TRIANGLES and a rest)
 // A warp's vertices: absolute (the general path), or packed 16-bit offsets
 // from the meshlet's corner (raster_meshlet_small), which needs no outcodes.
@@ -570,8 +566,13 @@ struct RasterSmem {
     uint8_t oc[kRasterWarps][MAX_MESHLET_UNIQUE_VERTICES];
     uint32_t micro[kRasterWarps][kMicroWords];
 };
+struct AlphaSmem {
+    AlphaVert av[MAX_MESHLET_UNIQUE_VERTICES];
+    AlphaRing ring;
+};
+static_assert(MAX_MESHLET_UNIQUE_VERTICES <= 64 && MAX_MESHLET_TRIANGLES <= 1 << 14, "AlphaRing::tri");
 struct RasterSmemAlpha : RasterSmem {
-    AlphaVert av[kRasterWarps][MAX_MESHLET_UNIQUE_VERTICES];
+    AlphaSmem alpha[kRasterWarps];
 };
 struct RasterSmemSmall : RasterSmem {
     __align__(16) RasterDraw draw[kRasterWarps][2][kMaxBatch];
@@ -597,16 +598,35 @@ struct MeshletWork {
 // ALPHA: the alpha-clip class (double sided, alpha tested per fragment).
 template <int KIND, bool ALPHA>
 __device__ __forceinline__ void raster_meshlet(const FrameDev& f, const MeshletWork w, RasterTune tune, SnapV* sv,
-                                               uint8_t* so, uint32_t* micro_words, AlphaVert* av, uint32_t lane,
+                                               uint8_t* so, uint32_t* micro_words, AlphaSmem* alpha, uint32_t lane,
                                                uint32_t& nfrag) {
     const uint32_t nv = w.nv, nt = w.nt, W = w.W, H = w.H;
     const MeshInfoRaster& mi = w.mi;
-    AlphaSrc as{av, 0u, H};
+    AlphaSrc as{};
     MeshInfoAlpha ma{};
     if (ALPHA) {
         ma = load_mesh_info_alpha(mesh_info_of(w.inst));
-        as.tex = ma.tex;
+        as = AlphaSrc{alpha->av, ma.tex, w.slot, alpha_size(W, H)};
     }
+    // the ring's entries (the same in every lane); a covered pixel joins them,
+    // and 32 of them are tested at once
+    uint32_t ring_first = 0, ring_n = 0;
+    auto join = [&](bool covered, uint32_t tri, int32_t px, int32_t py, float d) {
+        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, covered);
+        if (covered) {
+            const uint32_t i = (ring_first + ring_n + __popc(mask & ((1u << lane) - 1u))) & 63u;
+            alpha->ring.tri[i] = tri;
+            alpha->ring.pixel[i] = (uint32_t)px | (uint32_t)py << 16;
+            alpha->ring.depth[i] = d;
+        }
+        ring_n += __popc(mask);
+        if (ring_n < 32) return;
+        __syncwarp();
+        nfrag += alpha_fragments<KIND>(f, alpha->ring, ring_first, 32u, as, w.target, lane);
+        ring_first = (ring_first + 32u) & 63u;
+        ring_n -= 32u;
+        __syncwarp();
+    };
     // All of the meshlet's global loads are issued before any is used: the
     // micro-index words (at most 3 per lane; 4-byte aligned offsets, as the
     // meshletiser pads them), then both vertex indices of the lane, then both
@@ -642,7 +662,7 @@ __device__ __forceinline__ void raster_meshlet(const FrameDev& f, const MeshletW
         max_x = max(max_x, s.X);
         min_y = min(min_y, s.Y);
         max_y = max(max_y, s.Y);
-        if (ALPHA) av[j] = alpha_vert(c, ma, mi.flags, idx);
+        if (ALPHA) alpha->av[j] = alpha_vert(c, ma, mi.flags, idx);
     };
     if (v0) vertex(lane, idx0, pos0);
     if (v1) vertex(lane + 32u, idx1, pos1);
@@ -672,7 +692,7 @@ __device__ __forceinline__ void raster_meshlet(const FrameDev& f, const MeshletW
     const uint8_t* mic = reinterpret_cast<const uint8_t*>(micro_words);
     for (uint32_t base = w.part * 32u; base < nt; base += 32u * w.split) {
         const uint32_t t = base + lane;
-        bool medium = false, big = false;
+        bool small = false, medium = false, big = false;
         TriSetup st;
         if (t < nt) {
             const uint32_t m0 = mic[3 * t], m1 = mic[3 * t + 1], m2 = mic[3 * t + 2];
@@ -700,11 +720,11 @@ __device__ __forceinline__ void raster_meshlet(const FrameDev& f, const MeshletW
                         finish_setup(a, b, c, cr < 0 ? -cr : cr, box, LH_PACK_ID(t, w.slot), st);
                         if (ALPHA) {
                             st.bias |= kBiasAlpha;
-                            st.verts = m0 | (m1 << 8) | (m2 << 16);
+                            st.verts = m0 | m1 << 6 | m2 << 12 | t << 18;
                         }
                         uint32_t npx = (uint32_t)(st.px1 - st.px0 + 1) * (uint32_t)(st.py1 - st.py0 + 1);
                         if (npx <= tune.small_px) {
-                            if (ALPHA) nfrag += raster_lane_alpha<KIND>(f, st, w.target, W, as);
+                            if (ALPHA) small = true;  // below, the lanes' pixels together
                             else raster_lane<KIND>(st, w.target, W, nfrag);
                         } else if (npx <= medium_bin<KIND>(tune)) {
                             medium = true;
@@ -719,16 +739,52 @@ __device__ __forceinline__ void raster_meshlet(const FrameDev& f, const MeshletW
         // the occluder pass hold few meshlets with many big triangles each,
         // whose appends would otherwise queue on that one word
         if (__any_sync(0xFFFFFFFFu, big)) push_big_warp<KIND>(f, st, w.view, big, lane);
+        if (ALPHA && __any_sync(0xFFFFFFFFu, small)) {
+            // each lane walks its triangle's box, all of them in step
+            int32_t px = st.px0, py = st.py0;
+            EdgeSteps es{};
+            if (small && (st.bias & 8u)) es = edge_steps(st);
+            do {
+                float d = 0.0f;
+                const int32_t x = px, y = py;
+                bool covered = false;
+                if (small) {
+                    covered = (st.bias & 8u) ? cover_step(st, es, px - st.px0, py - st.py0, d) : cover(st, px, py, d);
+                    if (px++ == st.px1) {
+                        px = st.px0;
+                        small = py++ != st.py1;
+                    }
+                }
+                join(covered, st.verts, x, y, d);
+            } while (__any_sync(0xFFFFFFFFu, small));
+        }
         uint32_t mask = __ballot_sync(0xFFFFFFFFu, medium);
         while (mask) {
             int src = __ffs(mask) - 1;
             mask &= mask - 1;
             TriSetup b = shfl_setup(st, src);
-            if (ALPHA) nfrag += raster_warp_alpha<KIND>(f, b, w.target, W, lane, as);
-            else raster_warp<KIND>(b, w.target, W, lane, nfrag);
+            if (ALPHA) {
+                const uint32_t bw = (uint32_t)(b.px1 - b.px0 + 1), npx = bw * (uint32_t)(b.py1 - b.py0 + 1);
+                uint32_t rx = lane % bw, ry = lane / bw;
+                const uint32_t step_x = 32u % bw, step_y = 32u / bw;
+                for (uint32_t p = 0; p < npx; p += 32) {
+                    float d = 0.0f;
+                    const int32_t px = b.px0 + (int32_t)rx, py = b.py0 + (int32_t)ry;
+                    join(p + lane < npx && cover(b, px, py, d), b.verts, px, py, d);
+                    rx += step_x;
+                    ry += step_y;
+                    if (rx >= bw) rx -= bw, ry++;
+                }
+            } else {
+                raster_warp<KIND>(b, w.target, W, lane, nfrag);
+            }
         }
     }
     __syncwarp();
+    if (ALPHA && ring_n) {
+        nfrag += alpha_fragments<KIND>(f, alpha->ring, ring_first, ring_n, as, w.target, lane);
+        __syncwarp();
+    }
 }
 
 // A column-major matrix as row pairs: xy[c], zw[c] of column c.
@@ -1206,7 +1262,7 @@ __device__ __forceinline__ void first_window(const RasterWork& k, uint32_t gwarp
 // what the cull and the occlusion filter listed as kDrawGeneral.
 template <int KIND, bool ALPHA>
 __device__ __forceinline__ void raster_general_units(const FrameDev& f, uint32_t view_begin, RasterTune tune, uint32_t* claim_word,
-                                                     RasterSmem& sm, AlphaVert* av, uint32_t gwarp, uint32_t warp, uint32_t lane,
+                                                     RasterSmem& sm, AlphaSmem* alpha, uint32_t gwarp, uint32_t warp, uint32_t lane,
                                                      uint32_t& nfrag) {
     const RasterWork& work = sm.work[kLoopGeneral];
     const uint32_t first_slot = ALPHA ? f.max_draws : 0u;
@@ -1235,7 +1291,7 @@ __device__ __forceinline__ void raster_general_units(const FrameDev& f, uint32_t
             const MeshInfoRaster mi{rd.positions, rd.indices, rd.micro, 0, rd.bits >> 16};
             const MeshletWork w{view_begin + v, slot, part, 1u << work.split_shift, nv, nt, W, H, sm.view[v].target, (float)W * 0.5f,
                                 (float)H * 0.5f, &sm.vp[v], transform, mi, 0u, 0u, inst};
-            raster_meshlet<KIND, ALPHA>(f, w, tune, sm.v[warp].v, sm.oc[warp], sm.micro[warp], av, lane, nfrag);
+            raster_meshlet<KIND, ALPHA>(f, w, tune, sm.v[warp].v, sm.oc[warp], sm.micro[warp], alpha, lane, nfrag);
         }
         n = take_batch(sm, kLoopGeneral, first_slot, claimed, end, lane, v_lane, next);
         mine = next;
@@ -1368,12 +1424,12 @@ __device__ __forceinline__ void raster_setup(const FrameDev& f, uint32_t view_be
 // run out.  The alpha-clip class and the occluders, all on the general path:
 template <int KIND, bool ALPHA>
 __device__ void phase_raster_general(const FrameDev& f, uint32_t view_begin, uint32_t n_views, RasterTune tune, RasterSmem& sm,
-                                     AlphaVert (*s_av)[MAX_MESHLET_UNIQUE_VERTICES], uint32_t list) {
+                                     AlphaSmem* s_alpha, uint32_t list) {
     raster_setup<ALPHA>(f, view_begin, n_views, tune, sm, list);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t nfrag = 0;  // fragments this lane wrote
     raster_general_units<KIND, ALPHA>(f, view_begin, tune, &f.status[ALPHA ? kStRasterClaimAlpha : kStRasterClaimGeneral], sm,
-                                      ALPHA ? s_av[warp] : nullptr, blockIdx.x * (blockDim.x >> 5) + warp, warp, lane, nfrag);
+                                      ALPHA ? s_alpha + warp : nullptr, blockIdx.x * (blockDim.x >> 5) + warp, warp, lane, nfrag);
     count_fragments<KIND>(f, nfrag);
 }
 
@@ -1641,33 +1697,54 @@ __device__ __forceinline__ uint32_t upper_bound_warp(const uint32_t* base, uint3
     }
 }
 
-// The pixels [x0, x1] x [y0, y1] of an alpha-tested big triangle, one
-// column per lane (not inlined, as the other alpha paths).  The triangle is
-// passed as its queue entry: a reference to the caller's copy would keep
-// that copy in local memory on the opaque path too.
+// The pixels [x0, x1] x [y0, y1] of an alpha-tested big triangle by the whole
+// warp: covered ones, found 32 of a row at a time, wait in `wait` (64 x {pixel,
+// depth}) until 32 of them are tested at once.  Not inlined, as the other
+// alpha paths; the triangle is read from the queue, not handed over in
+// registers.
 template <int KIND>
 __device__ __noinline__ uint32_t raster_chunk_alpha(const FrameDev& f, const BigTri* entry, int32_t x0, int32_t x1,
-                                                    int32_t y0, int32_t y1, uint32_t lane) {
+                                                    int32_t y0, int32_t y1, uint32_t lane, uint2* wait) {
     const BigTri b = *entry;
     const ViewDev* vw = f.views + b.view;
     void* target = vw->target;
-    const uint32_t W = vw->width, H = vw->height;
+    const AlphaSize size = alpha_size(vw->width, vw->height);
     const AlphaTri at = alpha_tri_global(f, b.view, b.id);
     TriSetup t;
     t.X0 = b.X0; t.Y0 = b.Y0; t.X1 = b.X1; t.Y1 = b.Y1; t.X2 = b.X2; t.Y2 = b.Y2;
     t.z0 = b.z0; t.s1 = b.s1; t.s2 = b.s2;
     t.id = b.id;
     t.bias = b.bias;
-    uint32_t n = 0;
-    for (int32_t py = y0; py <= y1; py++)
-        for (int32_t px = x0 + (int32_t)lane; px <= x1; px += 32) {
-            float d;
-            if (cover(t, px, py, d) && alpha_pass(f, at, px, py, W, H)) {
-                write_fragment<KIND>(target, W, px, py, d, t.id);
+    uint32_t n = 0, first = 0, waiting = 0;
+    int32_t py = y0, px = x0;
+    for (;;) {
+        while (waiting < 32 && py <= y1) {
+            float d = 0.0f;
+            const int32_t x = px + (int32_t)lane;
+            const bool covered = x <= x1 && cover(t, x, py, d);
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, covered);
+            if (covered)
+                wait[(first + waiting + __popc(mask & ((1u << lane) - 1u))) & 63u] =
+                    make_uint2((uint32_t)x | (uint32_t)py << 16, f2u(d));
+            waiting += __popc(mask);
+            px += 32;
+            if (px > x1) px = x0, py++;
+        }
+        if (!waiting) return n;
+        const uint32_t now = min(waiting, 32u);
+        __syncwarp();
+        if (lane < now) {
+            const uint2 w = wait[(first + lane) & 63u];
+            const int32_t wx = (int32_t)(w.x & 0xFFFFu), wy = (int32_t)(w.x >> 16);
+            if (alpha_pass(f, at, wx, wy, size)) {
+                write_fragment<KIND>(target, size.W, wx, wy, u2f(w.y), t.id);
                 n++;
             }
         }
-    return n;
+        __syncwarp();
+        first = (first + now) & 63u;
+        waiting -= now;
+    }
 }
 
 // One warp per chunk of a big triangle (rows x columns of f.chunk_shift,
@@ -1680,13 +1757,13 @@ __device__ __noinline__ uint32_t raster_chunk_alpha(const FrameDev& f, const Big
 template <int KIND>
 __device__ __forceinline__ uint32_t raster_chunk(const FrameDev& f, const BigTri& b, const BigTri* entry, const ChunkSteps& ks,
                                                  int32_t x0, int32_t x1, int32_t y0, int32_t y1, uint32_t lane, void* target,
-                                                 uint32_t W) {
+                                                 uint32_t W, uint2* wait) {
     if (b.bias & kBiasAlpha) {
         if (edge_rejects(b.X1, b.Y1, b.X2, b.Y2, x0, x1, y0, y1, b.bias & 1u) ||
             edge_rejects(b.X2, b.Y2, b.X0, b.Y0, x0, x1, y0, y1, (b.bias >> 1) & 1u) ||
             edge_rejects(b.X0, b.Y0, b.X1, b.Y1, x0, x1, y0, y1, (b.bias >> 2) & 1u))
             return 0u;
-        return raster_chunk_alpha<KIND>(f, entry, x0, x1, y0, y1, lane);
+        return raster_chunk_alpha<KIND>(f, entry, x0, x1, y0, y1, lane, wait);
     }
     const uint32_t written = raster_chunk_runs<KIND>(f, b, ks, x0, x1, y0, y1, lane, target, W);
     return lane == 0 ? written : 0u;
@@ -1703,6 +1780,7 @@ struct BigSmem {
     // then two batches of whole triangles; kept here, not in registers
     __align__(16) BigTri tri[kRasterWarps][2 * kWholeBatch];
     ChunkSteps steps[kRasterWarps];
+    uint2 wait[kRasterWarps][64];  // covered pixels of alpha-tested triangles
 };
 
 // The chunks of the triangles too large to be taken whole, claimed in order.
@@ -1811,7 +1889,7 @@ __device__ __forceinline__ void raster_big_chunks(const FrameDev& f, BigSmem& sm
         c_next = c;
         cx += (int32_t)along;
         nfrag += raster_chunk<KIND>(f, b, f.big + t_idx, ks, x0, x1, y0, y1, lane, reinterpret_cast<void*>(sm.target[b.view]),
-                                    sm.width[b.view]);
+                                    sm.width[b.view], sm.wait[w]);
     }
     cp_async_wait_all();
     __syncwarp();
@@ -1853,7 +1931,7 @@ __device__ __forceinline__ void raster_big_whole(const FrameDev& f, BigSmem& sm,
             for (int32_t y0 = b.py0; y0 <= b.py1; y0 += 32)
                 for (int32_t x0 = b.px0; x0 <= b.px1; x0 += 256)
                     nfrag += raster_chunk<KIND>(f, b, f.big + i0 + k, ks, x0, min(b.px1, x0 + 255), y0, min(b.py1, y0 + 31), lane,
-                                                reinterpret_cast<void*>(sm.target[b.view]), sm.width[b.view]);
+                                                reinterpret_cast<void*>(sm.target[b.view]), sm.width[b.view], sm.wait[w]);
         }
         __syncwarp();
         i0 = next;
