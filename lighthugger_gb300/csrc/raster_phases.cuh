@@ -1791,7 +1791,11 @@ __device__ __forceinline__ void raster_big_chunks(const FrameDev& f, BigSmem& sm
     // out (the claim costs an atomic's and a search's round trips)
     const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);
     const uint32_t shift = LH_CHUNK_SHIFT - __clz(warps_total);
-    auto batch_of = [&](uint32_t left) { return min(max(left >> shift, 1u), (uint32_t)LH_CHUNK_BATCH); };
+    // (never fewer than the chunks beside one another that one set-up of runs
+    // serves, below: 1920 x 1080 before large walls 337 -> 317 us a frame;
+    // alpha-tested chunks go one by one and cost more: 423 -> 437 with foliage)
+    const uint32_t fewest = f.scene_alpha ? 1u : max(256u >> f.chunk_shift[KIND][1], 1u);
+    auto batch_of = [&](uint32_t left) { return min(max(left >> shift, fewest), (uint32_t)LH_CHUNK_BATCH); };
     const uint32_t first_batch = batch_of(total32);
     const uint32_t gwarp = blockIdx.x * (blockDim.x >> 5) + w;
     const uint64_t dyn_base = (uint64_t)warps_total * first_batch;
