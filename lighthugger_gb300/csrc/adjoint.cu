@@ -266,17 +266,6 @@ struct PixelOut {
     uint32_t idx[3];
 };
 
-// sign(dot(gn, normalize(vd))) as the IEEE arithmetic of the forward gives
-// it.  Its rounding moves the dot product by less than 2^-21 of the sum of
-// the terms' magnitudes and the undivided one's by less than 2^-22, so only
-// a sum of nearly cancelling terms (or of extreme ones) needs the divisions.
-__device__ __forceinline__ bool faces_away(f3 gn, f3 vd) {
-    const float x = gn.x * vd.x, y = gn.y * vd.y, z = gn.z * vd.z, d2 = dot(vd, vd);
-    const float s = (x + y) + z, m = (fabsf(x) + fabsf(y)) + fabsf(z);
-    if (fabsf(s) > m * (1.0f / 262144.0f) && fabsf(s) > 1e-30f && d2 > 1e-20f && d2 < 1e12f) return s < 0.0f;
-    return dot(gn, normalize(vd)) < 0.0f;
-}
-
 // Recompute the forward of pixel (x, y) from the visibility buffer and run
 // the surface half of the reverse pass of shade.cuh for the upstream
 // gradient at that pixel; fx, tri and st carry what the geometry half needs.

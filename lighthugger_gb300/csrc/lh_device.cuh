@@ -13,6 +13,7 @@
 
 #include <cstdint>
 
+#include "facing.cuh"
 #include "int_float.cuh"
 #include "lh/lh.h"
 
@@ -99,6 +100,8 @@ __device__ __forceinline__ int32_t wrap_texel(int32_t i, int32_t n) {
     const int32_t r = i % n;
     return r < 0 ? r + n : r;
 }
+
+__device__ __forceinline__ bool faces_away(f3 gn, f3 vd) { return faces_away(gn.x, gn.y, gn.z, vd.x, vd.y, vd.z); }
 
 // ------------------------------------------------------------------ scene access
 __device__ __forceinline__ const MeshInfo* mesh_info_of(const Instance* inst) {
