@@ -1,3 +1,5 @@
+// Signs of normalised dot products, decided without the normalisation.
+//
 // Whether a triangle with edge cross product n is seen from behind along v (the
 // vector to the camera): the sign of dot(n, normalize(v)) as IEEE arithmetic
 // gives it (dot = (x x' + y y') + z z'), mostly without the square root and the
@@ -26,6 +28,47 @@ LH_FACING_HD bool faces_away(float nx, float ny, float nz, float vx, float vy, f
     const float s = (x + y) + z, m = (fabsf(x) + fabsf(y)) + fabsf(z);
     if (fabsf(s) > m * (1.0f / 262144.0f) && fabsf(s) > 1e-30f && d2 > 1e-20f && d2 < 1e12f) return s < 0.0f;
     return faces_away_ieee(nx, ny, nz, vx, vy, vz);
+}
+
+// Whether a normal cone is seen from behind: dot(d', a') >= cutoff, where d' is
+// d normalised (`unit`: d as it is) and a' is a normalised `times` times, in IEEE
+// arithmetic.  Twelve divisions and roots lie behind that; their rounding, and
+// that of the approximate reciprocal roots here, moves the product by less
+// than 2^-20 of the sum of its terms' magnitudes, so they are only taken
+// nearer than 2^-18 to the cutoff, or for extreme lengths.
+LH_FACING_HD bool cone_behind_ieee(const float* d, const float* a, float cutoff, bool unit, int times) {
+    float x = a[0], y = a[1], z = a[2], u = d[0], v = d[1], w = d[2];
+    for (int i = 0; i < times; i++) {
+        const float l = sqrtf((x * x + y * y) + z * z);
+        x = x / l;
+        y = y / l;
+        z = z / l;
+    }
+    if (!unit) {
+        const float l = sqrtf((u * u + v * v) + w * w);
+        u = u / l;
+        v = v / l;
+        w = w / l;
+    }
+    return (u * x + v * y) + w * z >= cutoff;
+}
+
+LH_FACING_HD float rsqrt_near(float x) {
+#if defined(__CUDA_ARCH__)
+    return rsqrtf(x);
+#else
+    return 1.0f / sqrtf(x);
+#endif
+}
+
+LH_FACING_HD bool cone_behind(const float* d, const float* a, float cutoff, bool unit, int times) {
+    const float x = d[0] * a[0], y = d[1] * a[1], z = d[2] * a[2];
+    const float dd = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2], aa = (a[0] * a[0] + a[1] * a[1]) + a[2] * a[2];
+    const float q = unit ? rsqrt_near(aa) : rsqrt_near(aa) * rsqrt_near(dd);
+    const float c = ((x + y) + z) * q, m = ((fabsf(x) + fabsf(y)) + fabsf(z)) * q;
+    if (fabsf(c - cutoff) > m * (1.0f / 262144.0f) + 1e-20f && aa > 1e-16f && aa < 1e16f && dd > 1e-16f && dd < 1e16f)
+        return c > cutoff;
+    return cone_behind_ieee(d, a, cutoff, unit, times);
 }
 
 }  // namespace lh

@@ -243,13 +243,15 @@ __device__ __forceinline__ bool cull_bounding_sphere_shadows(const MiscStorage& 
 __device__ __forceinline__ bool cull_cone_perspective(const Uniforms& u, const Instance* inst, const lh_mat4& transform,
                                                       const Meshlet& ml) {
     f4 a4 = mul(transform, f4{ml.cone_apex.x, ml.cone_apex.y, ml.cone_apex.z, 1.0f});
-    f3 axis = normalize(mul3(inst->normal_transform, ld3(ml.cone_axis)));
-    return dot(normalize(f3{a4.x, a4.y, a4.z} - ld3(u.camera_pos)), normalize(axis)) >= ml.cone_cutoff;
+    const f3 axis = mul3(inst->normal_transform, ld3(ml.cone_axis)), to = f3{a4.x, a4.y, a4.z} - ld3(u.camera_pos);
+    const float d[3] = {to.x, to.y, to.z}, a[3] = {axis.x, axis.y, axis.z};
+    return cone_behind(d, a, ml.cone_cutoff, false, 2);
 }
 // culling.glsl:147-151
 __device__ __forceinline__ bool cull_cone_orthographic(const Uniforms& u, const Instance* inst, const Meshlet& ml) {
-    f3 axis = normalize(mul3(inst->normal_transform, ld3(ml.cone_axis)));
-    return dot(ld3(u.sun_dir), axis) >= ml.cone_cutoff;
+    const f3 axis = mul3(inst->normal_transform, ld3(ml.cone_axis));
+    const float d[3] = {u.sun_dir.x, u.sun_dir.y, u.sun_dir.z}, a[3] = {axis.x, axis.y, axis.z};
+    return cone_behind(d, a, ml.cone_cutoff, true, 1);
 }
 
 // ------------------------------------------------------------------ rasterisation rules
