@@ -2057,11 +2057,13 @@ __device__ __forceinline__ bool hiz_occluded(const ViewDev* vw, const lh_mat4& p
     for (int k = 0; k < 8; k++) {
         const float sa = (k & 1) ? 1.0f : -1.0f, sb = (k & 2) ? 1.0f : -1.0f, sd = (k & 4) ? 1.0f : -1.0f;
         const float cw = cc.w + sa * a.w + sb * b.w + sd * d.w;
-        if (!(cw > 1e-6f)) return false;
+        // (approximate reciprocals: their 2^-22 is far inside the margins below)
+        if (!(cw > 1e-6f && cw < 1e30f)) return false;
+        const float rw = __fdividef(1.0f, cw);
         const float cx = cc.x + sa * a.x + sb * b.x + sd * d.x;
         const float cy = cc.y + sa * a.y + sb * b.y + sd * d.y;
         const float cz = cc.z + sa * a.z + sb * b.z + sd * d.z;
-        const float px = (cx / cw) * hw + hw, py = (cy / cw) * hh + hh, pz = cz / cw;
+        const float px = (cx * rw) * hw + hw, py = (cy * rw) * hh + hh, pz = cz * rw;
         x0 = fminf(x0, px);
         x1 = fmaxf(x1, px);
         y0 = fminf(y0, py);
