@@ -7,11 +7,11 @@
 // point serves them: the caller passes the scene and the output sector, and
 // the only scratch the kernel needs -- the look-back words of its tiles and
 // the tile claim counter -- lives in a fixed array compiled into this library
-// (`g_cull_scratch` below, about 33 KB, held by every GPU that loads the
+// (`g_cull_scratch` below, about 8 KB, held by every GPU that loads the
 // library until the process exits).
 //
 // Limits and rules of use:
-//  - at most kNoAllocMaxTiles tiles of kInstTile instances (1,048,576
+//  - at most kNoAllocMaxTiles tiles of kCullTile instances (1,048,576
 //    instances); larger calls are rejected with LH_ERR_CAPACITY;
 //  - a call made outside stream capture looks up the device address of the
 //    array (cudaGetSymbolAddress) with the caller's device current and keeps
@@ -38,7 +38,7 @@ namespace cg = cooperative_groups;
 namespace lh {
 namespace {
 
-constexpr uint32_t kNoAllocMaxTiles = 4096;
+constexpr uint32_t kCullTile = 1024, kNoAllocMaxTiles = 1024, kNoAllocMaxInstances = kCullTile * kNoAllocMaxTiles;
 constexpr uint32_t kNoAllocWords = kNoAllocMaxTiles + 32;  // look-back words + the tile claim counter
 
 // The scratch of every call.  Host code must not use `g_cull_scratch`
@@ -53,21 +53,24 @@ std::atomic<unsigned long long*> g_scratch_ptr[kMaxDevices];
 // (cull_instances.comp:7-27 with prefix_sum.glsl:17-30): one instance per
 // thread, warp scans, decoupled look-back with bounded waits.
 //
-// Bound by HBM at the size of an open world (700,001 instances, 78 MB of
-// records: a floor of 12 us).  A tile's records are one bulk copy into shared
-// memory (28 KB, 7 blocks a SM: 200 KB in flight), so no thread's 112-byte
+// Bound, at the size of an open world (700,001 instances, 78 MB of records: a
+// floor of 12 us), by HBM and by the look-back, whose 32 predecessors a step
+// cross all tiles in flight: few large tiles.  A tile's records are one bulk
+// copy into shared memory (115 KB, 2 blocks a SM), so no thread's 112-byte
 // stride reaches the memory system, and a record is read from shared memory
 // without bank conflicts (28 words a lane: the 8 lanes of a 16-byte access
-// phase start 4 banks apart).  The look-back reads 32 predecessors at once.
-// 700,001 instances: 43 us, 52 with a thread's loads by itself and a look-back
-// of one predecessor at a time.
-__global__ void __launch_bounds__(kInstTile) k_cull_instances_noalloc(const Instance* instances, uint32_t n,
+// phase start 4 banks apart).  700,001 instances inside a graph: 35 us by tiles
+// of 256, 33 by 512, 28 by 1,024 (4,097: 4.4, 4.9 and 5.3); a call by itself 52
+// with each thread's own loads and a look-back of one predecessor at a time,
+// 35 now.
+__global__ void __launch_bounds__(kCullTile) k_cull_instances_noalloc(const Instance* instances, uint32_t n,
                                                                     const __grid_constant__ Uniforms u, uint8_t* sector,
                                                                     uint32_t capacity, uint32_t* flags_out,
                                                                     unsigned long long* scratch) {
-    __shared__ __align__(128) Instance s_inst[kInstTile];
+    extern __shared__ __align__(128) unsigned char s_dynamic[];
+    Instance* s_inst = reinterpret_cast<Instance*>(s_dynamic);  // [kCullTile]
     __shared__ __align__(8) uint64_t s_bar;
-    __shared__ uint64_t s_warp[kInstTile / 32];
+    __shared__ uint64_t s_warp[kCullTile / 32];
     __shared__ uint64_t s_excl;
     __shared__ uint32_t s_tile, s_flags;
     __shared__ SidePlanes s_planes;
@@ -80,16 +83,16 @@ __global__ void __launch_bounds__(kInstTile) k_cull_instances_noalloc(const Inst
         s_tile = tile;
         s_flags = 0u;
         if (tile < gridDim.x) {
-            const uint32_t bytes = min(n - tile * kInstTile, kInstTile) * (uint32_t)sizeof(Instance);
+            const uint32_t bytes = min(n - tile * kCullTile, kCullTile) * (uint32_t)sizeof(Instance);
             mbar_expect_tx(&s_bar, bytes);
-            bulk_load(s_inst, instances + (size_t)tile * kInstTile, bytes, &s_bar);
+            bulk_load(s_inst, instances + (size_t)tile * kCullTile, bytes, &s_bar);
         }
         s_planes = side_planes(u.perspective);
     }
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= gridDim.x) return;  // another call's claims: wrong results, but none out of range
-    const uint32_t i = tile * kInstTile + threadIdx.x;
+    const uint32_t i = tile * kCullTile + threadIdx.x;
     // (a copy that never lands: reported, the tile counts as empty)
     const bool landed = mbar_wait(&s_bar, 0u);
     if (!landed) atomicOr(&s_flags, LH_FLAG_TIMEOUT);
@@ -107,11 +110,11 @@ __global__ void __launch_bounds__(kInstTile) k_cull_instances_noalloc(const Inst
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        uint64_t sum = lane < kInstTile / 32 ? s_warp[lane] : 0ull;
+        uint64_t sum = lane < kCullTile / 32 ? s_warp[lane] : 0ull;
         const uint64_t own = sum;
         sum = warp_incl_scan(sum);
-        if (lane < kInstTile / 32) s_warp[lane] = sum - own;
-        const uint64_t run = __shfl_sync(0xFFFFFFFFu, sum, kInstTile / 32 - 1);
+        if (lane < kCullTile / 32) s_warp[lane] = sum - own;
+        const uint64_t run = __shfl_sync(0xFFFFFFFFu, sum, kCullTile / 32 - 1);
         const uint64_t excl = lookback_warp(status, tile, run, &s_flags);
         if (lane == 0) {
             s_excl = excl;
@@ -142,7 +145,7 @@ __global__ void __launch_bounds__(kInstTile) k_cull_instances_noalloc(const Inst
 // the call is one launch.  Bound by latency and, at one block, by issue (the
 // square roots and divisions of 32 warps on one SM): inside a graph 1,024
 // instances take 2.3 us by 8 blocks, 4.1 by one, 4.4 cleared and by tiles; 4,096
-// take 3.6 and 4,097, by tiles, 5.1.  A call by itself: 4.1 us, 9.2 before.
+// take 3.6 and 4,097, by tiles, 5.3.  A call by itself: 4.1 us, 9.2 before.
 constexpr uint32_t kSmallBlocks = 8, kSmallThreads = 512, kSmallInstances = kSmallBlocks * kSmallThreads;
 __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads) k_cull_instances_noalloc_small(
     const Instance* instances, uint32_t n, const __grid_constant__ Uniforms u, uint8_t* sector, uint32_t capacity,
@@ -233,8 +236,8 @@ extern "C" lh_status lh_cull_instances_noalloc(const Instance* d_instances, uint
     using namespace lh;
     if (!host_uniforms || !d_sector || (n_instances && !d_instances)) return LH_ERR_INVALID_ARGUMENT;
     if (((uintptr_t)d_instances & 15) || ((uintptr_t)d_sector & 7)) return LH_ERR_INVALID_ARGUMENT;
-    const uint32_t tiles = (n_instances + kInstTile - 1) / kInstTile;
-    if (tiles > kNoAllocMaxTiles) return LH_ERR_CAPACITY;  // more than 1,048,576 instances
+    const uint32_t tiles = (n_instances + kCullTile - 1) / kCullTile;
+    if (n_instances > kNoAllocMaxInstances) return LH_ERR_CAPACITY;  // more than 1,048,576 instances
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     unsigned long long* scratch = nullptr;
     lh_status st = scratch_for_current_device(s, &scratch);
@@ -251,7 +254,10 @@ extern "C" lh_status lh_cull_instances_noalloc(const Instance* d_instances, uint
         if (cudaMemsetAsync(d_sector, 0, 8, s) != cudaSuccess) return LH_ERR_CUDA;
         return LH_OK;
     }
-    k_cull_instances_noalloc<<<tiles, kInstTile, 0, s>>>(d_instances, n_instances, *host_uniforms, d_sector, capacity,
+    constexpr uint32_t kShared = kCullTile * (uint32_t)sizeof(Instance);
+    if (cudaFuncSetAttribute(k_cull_instances_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShared) != cudaSuccess)
+        return LH_ERR_CUDA;
+    k_cull_instances_noalloc<<<tiles, kCullTile, kShared, s>>>(d_instances, n_instances, *host_uniforms, d_sector, capacity,
                                                         d_flags, scratch);
     return cudaGetLastError() == cudaSuccess ? LH_OK : LH_ERR_CUDA;
 }

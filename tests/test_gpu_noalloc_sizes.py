@@ -1,7 +1,7 @@
 """lh_cull_instances_noalloc over the sizes where its two kernels and their
-tiles end: one cluster of 8 blocks up to 4,096 instances, 256-instance tiles with a look-back
-above.  Entries stand in instance order, so the sector of the first n instances
-is the beginning of the sector of all of them."""
+tiles end: one cluster of 8 blocks up to 4,096 instances, 1,024-instance tiles
+with a look-back above.  Entries stand in instance order, so the sector of the
+first n instances is the beginning of the sector of all of them."""
 import ctypes as C
 
 import numpy as np
@@ -10,7 +10,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 TOTAL = 20011
-SIZES = (1, 31, 32, 33, 249, 255, 256, 257, 1023, 1024, 1025, 3073, 4095, 4096, 4097, 4351, 4352, 4353, 8191, 8193, 16641, TOTAL)
+SIZES = (1, 31, 32, 33, 249, 255, 256, 257, 1023, 1024, 1025, 3073, 4095, 4096, 4097, 4351, 4352, 4353, 8191, 5119, 5120, 5121, 8191, 8193, 16641, TOTAL)
 
 
 def test_noalloc_cull_sizes(native):
