@@ -159,15 +159,6 @@ __device__ __forceinline__ float pow5f(float x) {
     const float x2 = x * x;
     return x2 * x2 * x;
 }
-// v / |v| by a Newton step on the approximate reciprocal square root r of the
-// fused sum of squares, its correction added to v r before the one rounding:
-// relative error at most 1.52e-7, 2.63e-8 on average (an IEEE root and three
-// divisions, without fusing: 1.84e-7 and 3.26e-8; over 2.6e8 random vectors).
-__device__ __forceinline__ f3 near_normalize(f3 v) {
-    const float d = __fmaf_rn(v.x, v.x, __fmaf_rn(v.y, v.y, v.z * v.z)), r = rsqrtf(d);
-    const float c = 0.5f * r * __fmaf_rn(-d * r, r, 1.0f);
-    return f3{__fmaf_rn(v.x, r, v.x * c), __fmaf_rn(v.y, r, v.y * c), __fmaf_rn(v.z, r, v.z * c)};
-}
 __device__ __forceinline__ f3 fast_normalize(f3 v) { return v * rsqrtf(dot(v, v)); }
 __device__ __forceinline__ float F_Schlick1(float u, float f0, float f90) { return f0 + (f90 - f0) * pow5f(1.0f - u); }
 __device__ __forceinline__ float Fd_Burley(float NoV, float NoL, float LoH, float rough) {
@@ -494,11 +485,11 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& f, uint32_t x, uin
     const f3 world{dot(f3{pa.x, pb.x, pc.x}, bary.lambda), dot(f3{pa.y, pb.y, pc.y}, bary.lambda),
                    dot(f3{pa.z, pb.z, pc.z}, bary.lambda)};
     f2 uv{dot(us, bary.lambda) + mi.texture_offset.x, dot(vs, bary.lambda) + mi.texture_offset.y};
-    const f3 to_camera = ld3(u.camera_pos) - world;
+    const f3 view_vector = normalize(ld3(u.camera_pos) - world);
     f3 normal{interp_deriv(bary, na.x, nb.x, nc.x).x, interp_deriv(bary, na.y, nb.y, nc.y).x,
               interp_deriv(bary, na.z, nb.z, nc.z).x};
     normal = fast_normalize(mul3(inst->normal_transform, normal));
-    if (faces_away(cross(pb - pa, pc - pa), to_camera)) normal = -normal;
+    if (dot(cross(pb - pa, pc - pa), view_vector) < 0.0f) normal = -normal;
     // materials first (they need the geometry the shadow code below does not,
     // so its registers free up early; the order changes no result)
     Tex4 bc = sample_repeat(f, mi.base_tex, uv);
@@ -551,7 +542,7 @@ __device__ __forceinline__ void resolve_pixel(const FrameDev& f, uint32_t x, uin
     float sun_intensity = kPi * shadow_sum;
     // Uniforms.sun_intensity is the light colour (1,1,1 in the reference, whose
     // shaders never read it; main.cpp:649): a multiply by 1 leaves every bit.
-    f3 sun = (BRDF(near_normalize(to_camera), ld3(u.sun_dir), normal, roughness, metallic, base, alpha) * sun_intensity) *
+    f3 sun = (BRDF(view_vector, ld3(u.sun_dir), normal, roughness, metallic, base, alpha) * sun_intensity) *
              ld3(u.sun_intensity);
     f3 o = sun + ambient;
     if (u.debug == 4) o = clock_view(*clock_slot);
