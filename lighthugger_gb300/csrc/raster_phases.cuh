@@ -1837,13 +1837,24 @@ __device__ __forceinline__ void raster_big_chunks(const FrameDev& f, BigSmem& sm
             // another triangle, by a 32-ary search of the bases; often the
             // copied-ahead next entry
             __syncwarp();  // every lane is done with the current slot
-            const uint32_t first = upper_bound_warp(f.big_base, t_end ? t_idx : 0u, ntri, c, lane);
-            if (first == 0) {
-                c++;
-                continue;
+            uint32_t i = pre_idx, base = t_end;
+            bool next = false;
+            if (c == t_end && pre_idx != 0xFFFFFFFFu) {
+                // bases ascend without gaps: the chunk after a triangle's last is
+                // the next entry's first, unless that one is taken whole
+                cp_async_wait_all();
+                __syncwarp();
+                next = !(s_tri[slot ^ 1u].bias & kBiasWhole);
             }
-            const uint32_t i = first - 1;
-            const uint32_t base = f.big_base[i];
+            if (!next) {
+                const uint32_t first = upper_bound_warp(f.big_base, t_end ? t_idx : 0u, ntri, c, lane);
+                if (first == 0) {
+                    c++;
+                    continue;
+                }
+                i = first - 1;
+                base = f.big_base[i];
+            }
             if (i == pre_idx) {
                 cp_async_wait_all();
                 __syncwarp();
