@@ -1790,7 +1790,9 @@ __device__ __forceinline__ void raster_big_chunks(const FrameDev& f, BigSmem& sm
     // static first batch per warp, then claims that shrink as the chunks run
     // out (the claim costs an atomic's and a search's round trips)
     const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);
-    const uint32_t shift = LH_CHUNK_SHIFT - __clz(warps_total);
+    // (a chunk of an alpha-tested triangle costs several times an opaque one's:
+    // claims a quarter as large, 2258 x 406 close to foliage 1305 -> 1184 us)
+    const uint32_t shift = LH_CHUNK_SHIFT - __clz(warps_total) + (f.scene_alpha ? 2u : 0u);
     // (never fewer than the chunks beside one another that one set-up of runs
     // serves, below: 1920 x 1080 before large walls 337 -> 317 us a frame;
     // alpha-tested chunks go one by one and cost more: 423 -> 437 with foliage)
