@@ -253,7 +253,7 @@ typedef struct lh_tuning {
                                  first, the hierarchical depth of what they wrote is built, and every other
                                  meshlet whose sphere lies behind it is skipped (no counterpart in the
                                  reference; results identical).  0: one pass, no occlusion test; so are
-                                 opaque scenes of at most 32,768 meshlets (times the visibility views) */
+                                 scenes of at most 32,768 meshlets (times the visibility views) */
     uint32_t chunk_rows[2];   /* pixel rows of a big-triangle chunk (one warp) in the visibility / shadow
                                  pass: 4, 8, 16 or 32 */
     uint32_t chunk_cols[2];   /* its columns: 32, 64, 128 or 256 */

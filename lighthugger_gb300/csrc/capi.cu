@@ -269,19 +269,19 @@ size_t reset_bytes_for(const lh_ctx* c) {
 }
 
 // The occluder threshold of a frame of n_views views (4 of them cascades).
-// The two-pass raster's four launches cost 14 to 30 us a frame; rasterising
-// what they would have skipped costs about 1 ns a meshlet, so opaque scenes
-// of at most kOnePassMeshlets meshlets, counted once per visibility view, take
-// one pass.  Measured by launches: 3,840 meshlets at 640 x 360 105 -> 91 us,
-// 15,360 at 1280 x 720 116 -> 102, 35,145 (two thirds of the visible ones
-// hidden) 189 -> 161, 44,496 258 -> 232, 145,845 290 -> 262; the other way
-// round 595,594 at 1920 x 1080 336 -> 395 and 498 -> 562, and with
-// alpha-tested meshes, whose hidden pixels cost a texture sample each, 88,261
-// 459 -> 564.  The line lies where no view can gain 30 us.
+// The two-pass raster's four launches cost 13 to 30 us a frame; rasterising
+// what they would have skipped costs about 1 ns a meshlet, 5 an alpha-tested
+// one, so scenes of at most kOnePassMeshlets meshlets, counted once per
+// visibility view, take one pass.  Measured by launches: 3,840 meshlets at 640 x
+// 360 105 -> 91 us, 15,360 at 1280 x 720 116 -> 102, 35,145 (two thirds of the
+// visible ones hidden) 189 -> 161, 44,496 258 -> 232, 145,845 290 -> 262; half
+// of them alpha-tested: 1,200 101 -> 89 us, 15,360 189 -> 174, 25,920 183 ->
+// 168, 27,993 283 -> 267.  The other way round 595,594 at 1920 x 1080 336 ->
+// 395 and 498 -> 562, and with alpha-tested ones 88,261 459 -> 564.
 constexpr uint64_t kOnePassMeshlets = 32768;
 uint32_t occlusion_px_of(const lh_ctx* c, uint32_t n_views) {
     const uint64_t visibility_views = n_views > 4 ? n_views - 4 : 1;
-    return !c->scene_alpha && c->scene_meshlets * visibility_views <= kOnePassMeshlets ? 0u : c->tuning.occlusion_px;
+    return c->scene_meshlets * visibility_views <= kOnePassMeshlets ? 0u : c->tuning.occlusion_px;
 }
 
 FrameDev frame_dev(const lh_ctx* c, uint32_t n_views, uint32_t n_instances) {
