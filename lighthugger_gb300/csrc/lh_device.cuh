@@ -13,6 +13,7 @@
 
 #include <cstdint>
 
+#include "big_queue.cuh"
 #include "facing.cuh"
 #include "int_float.cuh"
 #include "lh/lh.h"
@@ -318,8 +319,6 @@ struct TriSetup {
                     // bit4 (kBiasAlpha): alpha-tested
     uint32_t verts;  // alpha-tested: meshlet vertices m0 | m1 << 6 | m2 << 12, triangle << 18
 };
-constexpr uint32_t kBiasAlpha = 16u;
-constexpr uint32_t kBiasWhole = 32u;  // BigTri: taken whole by one warp, not by chunks
 
 __device__ __forceinline__ bool top_left(int32_t ax, int32_t ay, int32_t bx, int32_t by) {
     int32_t dy = by - ay, dx = bx - ax;

@@ -263,45 +263,21 @@ __device__ __forceinline__ void load_transform(const Instance* inst, lh_mat4& m)
 // (the packed single-pass append of prefix_sum.glsl:17-30): the triangle's
 // index and its first chunk come from the same word, so chunk bases ascend
 // with the index and the chunk kernel finds a chunk's triangle by binary search.
-// An opaque triangle of at most kWholeChunks chunks is queued whole
-// (kBiasWhole) and adds no chunk: the chunk kernel takes those by their
-// index, without a search (alpha-tested pixels cost several times an opaque
-// one: those stay in chunks).  (Entries without chunks keep the search exact: the last entry
+// Opaque triangles of at most kWholeChunks chunks are queued whole
+// (big_queue.cuh): the chunk kernel takes those by their index, without a
+// search (alpha-tested pixels cost several times an opaque one: those stay in
+// chunks).  (Entries without chunks keep the search exact: the last entry
 // whose base is at most a chunk's number is the one that holds it.)
-#ifndef LH_WHOLE_CHUNKS
-#define LH_WHOLE_CHUNKS 2
-#endif
-constexpr unsigned long long kWholeChunks = LH_WHOLE_CHUNKS;
 template <int KIND>
 __device__ __forceinline__ unsigned long long box_chunks(const FrameDev& f, uint32_t w, uint32_t h) {  // extents - 1
     return (unsigned long long)((w >> f.chunk_shift[KIND][1]) + 1u) * ((h >> f.chunk_shift[KIND][0]) + 1u);
-}
-__device__ __forceinline__ bool taken_whole(unsigned long long n, bool alpha) { return n <= kWholeChunks && !alpha; }
-// The packed word of a triangle of n chunks.
-__device__ __forceinline__ unsigned long long queue_word(unsigned long long n, bool alpha) {
-    return (1ull << 40) | (taken_whole(n, alpha) ? 0ull : n);
 }
 // Store the queue entry of a triangle of n chunks whose packed word (before
 // its own addition) is `old`.
 __device__ void store_big(const FrameDev& f, const TriSetup& t, uint32_t view, unsigned long long old,
                           unsigned long long n) {
-    const uint64_t idx = old >> 40, base = old & ((1ull << 40) - 1);
-    if (idx >= f.big_cap || base + n > 0xFFFFFFFFull) {
+    if (!store_queue_entry(f.big, f.big_base, f.big_cap, t, view, old, n))
         atomicOr(&f.status[kStFlags], LH_FLAG_QUEUE_OVERFLOW);
-        return;
-    }
-    BigTri e;
-    e.X0 = t.X0; e.Y0 = t.Y0; e.X1 = t.X1; e.Y1 = t.Y1; e.X2 = t.X2; e.Y2 = t.Y2;
-    e.z0 = t.z0; e.s1 = t.s1; e.s2 = t.s2;
-    e.id = t.id;
-    e.view = view;
-    e.bias = t.bias | (taken_whole(n, t.bias & kBiasAlpha) ? kBiasWhole : 0u);
-    e.px0 = t.px0;
-    e.px1 = t.px1;
-    e.py0 = t.py0;
-    e.py1 = t.py1;
-    f.big[idx] = e;
-    f.big_base[idx] = (uint32_t)base;
 }
 // One thread's triangle.
 template <int KIND>
@@ -313,8 +289,9 @@ __device__ void push_big(const FrameDev& f, const TriSetup& t, uint32_t view) {
 }
 // Called by the whole warp: lanes with n != 0 append their triangle of n
 // chunks with one atomic per warp (a warp scan of the lanes' words gives each
-// lane the running total below it).  The word's low 40 bits cannot carry into
-// the count: a sum reaching 2^32 chunks is flagged and dropped.
+// lane the running total below it).  A sum reaching 2^32 chunks is flagged and
+// dropped; the word's low 40 bits hold it up to half a million triangles
+// that each fill a 16,384 x 16,384 view in the smallest chunks.
 __device__ __forceinline__ unsigned long long reserve_big_warp(const FrameDev& f, unsigned long long n, bool alpha, uint32_t lane) {
     const unsigned long long mine = n ? queue_word(n, alpha) : 0ull;
     unsigned long long incl = mine;
