@@ -16,15 +16,28 @@ namespace lh {
 constexpr uint32_t kBiasAlpha = 16u;  // TriSetup / BigTri bias: alpha-tested
 constexpr uint32_t kBiasWhole = 32u;  // BigTri: taken whole by one warp, not by chunks
 
-// An opaque triangle of at most kWholeChunks chunks is queued whole
-// (kBiasWhole) and adds no chunk.
+// An opaque triangle of at most this many chunks is queued whole (kBiasWhole)
+// and adds no chunk.  KIND: the pass (0 visibility, 1 shadow).  One warp takes
+// a whole triangle, at the launch's end: two visibility chunks (16 x 128 by
+// default) are still one or two set-ups of rows, two shadow chunks (32 x 64) up
+// to 4,096 pixels, which kept the cascades' launch waiting for a few warps.
+// Shadow raster at limits 0 / 1 / 2 / 3, us: 1080p frame of the benchmark 75.7 /
+// 75.8 / 81.9 / 84.0, before walls 210.9 / 186-188 / 192.5 / 211-213, 512 x 512
+// training step 172-174 / 155.6 / 161.8 / 176.1; visibility raster at 1 / 2
+// before walls: 163.5 / 149.2.
 #ifndef LH_WHOLE_CHUNKS
 #define LH_WHOLE_CHUNKS 2
 #endif
-constexpr uint64_t kWholeChunks = LH_WHOLE_CHUNKS;
-LH_BQ_HD bool taken_whole(uint64_t n, bool alpha) { return n <= kWholeChunks && !alpha; }
+#ifndef LH_SHADOW_WHOLE_CHUNKS
+#define LH_SHADOW_WHOLE_CHUNKS 1
+#endif
+template <int KIND> LH_BQ_HD bool taken_whole(uint64_t n, bool alpha) {
+    return n <= (KIND == 0 ? LH_WHOLE_CHUNKS : LH_SHADOW_WHOLE_CHUNKS) && !alpha;
+}
 // What a triangle of n chunks adds to the counter.
-LH_BQ_HD uint64_t queue_word(uint64_t n, bool alpha) { return (1ull << 40) | (taken_whole(n, alpha) ? 0ull : n); }
+template <int KIND> LH_BQ_HD uint64_t queue_word(uint64_t n, bool alpha) {
+    return (1ull << 40) | (taken_whole<KIND>(n, alpha) ? 0ull : n);
+}
 
 // Write the entry of a triangle `t` of n chunks whose counter (before its own
 // addition) is `old`; false when it does not fit and is dropped.  The chunk
@@ -33,7 +46,7 @@ LH_BQ_HD uint64_t queue_word(uint64_t n, bool alpha) { return (1ull << 40) | (ta
 // as one that covers nothing: whole (no chunk is looked up in it), with an
 // empty box, and a base above every chunk number so that the bases stay in
 // order.  Left as it was, the slot would hold a triangle of an earlier pass.
-template <class Big, class Setup>
+template <int KIND, class Big, class Setup>
 LH_BQ_HD bool store_queue_entry(Big* big, uint32_t* big_base, uint32_t cap, const Setup& t, uint32_t view, uint64_t old,
                                 uint64_t n) {
     const uint64_t idx = old >> 40, base = old & ((1ull << 40) - 1);
@@ -44,7 +57,7 @@ LH_BQ_HD bool store_queue_entry(Big* big, uint32_t* big_base, uint32_t cap, cons
     e.z0 = t.z0; e.s1 = t.s1; e.s2 = t.s2;
     e.id = t.id;
     e.view = view;
-    e.bias = !fits ? kBiasWhole : t.bias | (taken_whole(n, t.bias & kBiasAlpha) ? kBiasWhole : 0u);
+    e.bias = !fits ? kBiasWhole : t.bias | (taken_whole<KIND>(n, t.bias & kBiasAlpha) ? kBiasWhole : 0u);
     e.px0 = t.px0;
     e.px1 = t.px1;
     e.py0 = fits ? t.py0 : 1;

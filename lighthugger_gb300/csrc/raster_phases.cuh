@@ -263,8 +263,8 @@ __device__ __forceinline__ void load_transform(const Instance* inst, lh_mat4& m)
 // (the packed single-pass append of prefix_sum.glsl:17-30): the triangle's
 // index and its first chunk come from the same word, so chunk bases ascend
 // with the index and the chunk kernel finds a chunk's triangle by binary search.
-// Opaque triangles of at most kWholeChunks chunks are queued whole
-// (big_queue.cuh): the chunk kernel takes those by their index, without a
+// Opaque triangles of one or two chunks are queued whole (taken_whole,
+// big_queue.cuh): the chunk kernel takes those by their index, without a
 // search (alpha-tested pixels cost several times an opaque one: those stay in
 // chunks).  (Entries without chunks keep the search exact: the last entry
 // whose base is at most a chunk's number is the one that holds it.)
@@ -274,9 +274,10 @@ __device__ __forceinline__ unsigned long long box_chunks(const FrameDev& f, uint
 }
 // Store the queue entry of a triangle of n chunks whose packed word (before
 // its own addition) is `old`.
+template <int KIND>
 __device__ void store_big(const FrameDev& f, const TriSetup& t, uint32_t view, unsigned long long old,
                           unsigned long long n) {
-    if (!store_queue_entry(f.big, f.big_base, f.big_cap, t, view, old, n))
+    if (!store_queue_entry<KIND>(f.big, f.big_base, f.big_cap, t, view, old, n))
         atomicOr(&f.status[kStFlags], LH_FLAG_QUEUE_OVERFLOW);
 }
 // One thread's triangle.
@@ -284,16 +285,17 @@ template <int KIND>
 __device__ void push_big(const FrameDev& f, const TriSetup& t, uint32_t view) {
     const unsigned long long n = box_chunks<KIND>(f, (uint32_t)(t.px1 - t.px0), (uint32_t)(t.py1 - t.py0));
     const unsigned long long old =
-        atomicAdd(reinterpret_cast<unsigned long long*>(f.status + kStBigPacked), queue_word(n, t.bias & kBiasAlpha));
-    store_big(f, t, view, old, n);
+        atomicAdd(reinterpret_cast<unsigned long long*>(f.status + kStBigPacked), queue_word<KIND>(n, t.bias & kBiasAlpha));
+    store_big<KIND>(f, t, view, old, n);
 }
 // Called by the whole warp: lanes with n != 0 append their triangle of n
 // chunks with one atomic per warp (a warp scan of the lanes' words gives each
 // lane the running total below it).  A sum reaching 2^32 chunks is flagged and
 // dropped; the word's low 40 bits hold it up to half a million triangles
 // that each fill a 16,384 x 16,384 view in the smallest chunks.
+template <int KIND>
 __device__ __forceinline__ unsigned long long reserve_big_warp(const FrameDev& f, unsigned long long n, bool alpha, uint32_t lane) {
-    const unsigned long long mine = n ? queue_word(n, alpha) : 0ull;
+    const unsigned long long mine = n ? queue_word<KIND>(n, alpha) : 0ull;
     unsigned long long incl = mine;
 #pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {
@@ -307,8 +309,8 @@ __device__ __forceinline__ unsigned long long reserve_big_warp(const FrameDev& f
 template <int KIND>
 __device__ void push_big_warp(const FrameDev& f, const TriSetup& t, uint32_t view, bool big, uint32_t lane) {
     const unsigned long long n = big ? box_chunks<KIND>(f, (uint32_t)(t.px1 - t.px0), (uint32_t)(t.py1 - t.py0)) : 0ull;
-    const unsigned long long old = reserve_big_warp(f, n, t.bias & kBiasAlpha, lane);
-    if (big) store_big(f, t, view, old, n);
+    const unsigned long long old = reserve_big_warp<KIND>(f, n, t.bias & kBiasAlpha, lane);
+    if (big) store_big<KIND>(f, t, view, old, n);
 }
 
 // Sutherland-Hodgman against w-z, z, g*w-x, g*w+x, g*w-y, g*w+y >= 0.
@@ -918,14 +920,14 @@ __device__ __forceinline__ uint32_t raster_large(const FrameDev& f, const Meshle
             if (!medium) chunks = box_chunks<KIND>(f, w, h);
         }
         if (__any_sync(0xFFFFFFFFu, chunks != 0)) {
-            const unsigned long long old = reserve_big_warp(f, chunks, false, lane);
+            const unsigned long long old = reserve_big_warp<KIND>(f, chunks, false, lane);
             if (chunks) {
                 const uint32_t t = mv.p.large[base + lane];
                 SmallTri s;
                 small_tri<KIND>(mv, mic, t, bx, by, vt, s);
                 TriSetup st;
                 setup_of<KIND>(s, t, slot, bx, by, st);
-                store_big(f, st, view, old, chunks);
+                store_big<KIND>(f, st, view, old, chunks);
             }
         }
         uint32_t mask = __ballot_sync(0xFFFFFFFFu, medium);

@@ -24,10 +24,12 @@ struct Big {
     int32_t px0, px1, py0, py1;
 };
 
-int main() {
-    std::mt19937_64 rng(5);
-    long long entries = 0, dropped = 0, bad = 0;
-    for (int it = 0; it < 400; it++) {
+long long entries = 0, dropped = 0, bad = 0;
+
+// KIND: the pass.
+template <int KIND> void run(uint64_t seed) {
+    std::mt19937_64 rng(seed);
+    for (int it = 0; it < 200; it++) {
         const uint32_t cap = 1 + (uint32_t)(rng() % 6000), pushes = 1 + (uint32_t)(rng() % 7000);
         // every other queue: the smallest chunks and boxes of nearly 16,384 pixels a side
         const bool past = it & 1;
@@ -48,8 +50,8 @@ int main() {
             t.bias = rng() % 4 == 0 ? lh::kBiasAlpha : 0u;
             const uint64_t n = (uint64_t)(((uint32_t)(t.px1 - t.px0) >> cs) + 1) * (((uint32_t)(t.py1 - t.py0) >> rs) + 1);
             const uint64_t old = word;
-            word += lh::queue_word(n, t.bias & lh::kBiasAlpha);
-            const bool ok = lh::store_queue_entry(big.data(), base.data(), cap, t, 3u, old, n);
+            word += lh::queue_word<KIND>(n, t.bias & lh::kBiasAlpha);
+            const bool ok = lh::store_queue_entry<KIND>(big.data(), base.data(), cap, t, 3u, old, n);
             const bool want = k < cap && (old & ((1ull << 40) - 1)) + n <= 0xFFFFFFFFull;
             if (ok != want) bad++;
             sent.push_back(t);
@@ -78,6 +80,17 @@ int main() {
             if (taken && !fits[at - 1]) bad++;
         }
     }
+}
+
+int main() {
+    run<0>(5);
+    run<1>(6);
+    // whole up to two visibility chunks and one shadow chunk, alpha-tested never
+    for (uint64_t n = 1; n < 5; n++)
+        for (int alpha = 0; alpha < 2; alpha++) {
+            if ((lh::queue_word<0>(n, alpha) & 0xFFFF) != (n <= 2 && !alpha ? 0 : n)) bad++;
+            if ((lh::queue_word<1>(n, alpha) & 0xFFFF) != (n <= 1 && !alpha ? 0 : n)) bad++;
+        }
     std::printf("entries %lld dropped %lld bad %lld\n", entries, dropped, bad);
     return bad != 0 || dropped == 0;
 }
