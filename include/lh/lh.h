@@ -240,6 +240,7 @@ lh_status lh_read_status(lh_ctx* ctx, lh_device_status* out);
 #define LH_SCHEDULE_PER_STAGE 1  /* one launch per stage, each over all views of a kind */
 #define LH_SCHEDULE_PERSISTENT 2 /* cull + raster of all views in one cooperative launch */
 #define LH_SCHEDULE_PER_VIEW 3   /* each view's cull and raster launched on its own (the reference's per-cascade loop) */
+#define LH_OCCLUSION_PX_DEFAULT 128u /* lh_create's lh_tuning.occlusion_px */
 typedef struct lh_tuning {
     uint32_t small_px;        /* a lane rasterises triangles whose bbox has <= small_px pixels */
     uint32_t medium_px;       /* the warp rasterises up to medium_px; larger go to chunks (chunk_rows x
@@ -252,8 +253,10 @@ typedef struct lh_tuning {
                                  bounding sphere projects to a radius above this many pixels are drawn
                                  first, the hierarchical depth of what they wrote is built, and every other
                                  meshlet whose sphere lies behind it is skipped (no counterpart in the
-                                 reference; results identical).  0: one pass, no occlusion test; so are
-                                 scenes of at most 32,768 meshlets (times the visibility views) */
+                                 reference; results identical).  0: one pass, no occlusion test.  The
+                                 default, LH_OCCLUSION_PX_DEFAULT, draws scenes of at most 32,768 meshlets
+                                 (times the visibility views) in one pass; any other value is taken as
+                                 it is */
     uint32_t chunk_rows[2];   /* pixel rows of a big-triangle chunk (one warp) in the visibility / shadow
                                  pass: 4, 8, 16 or 32 */
     uint32_t chunk_cols[2];   /* its columns: 32, 64, 128 or 256 */

@@ -268,7 +268,8 @@ size_t reset_bytes_for(const lh_ctx* c) {
     return align_up(kStWords * 4, 256) + per_view * c->max_views;
 }
 
-// The occluder threshold of a frame of n_views views (4 of them cascades).
+// The occluder threshold of a frame of n_views views (4 of them cascades): the
+// tuning's, or what suits the scene where it is the default.
 // The two-pass raster's four launches cost 13 to 30 us a frame; rasterising
 // what they would have skipped costs about 1 ns a meshlet, 5 an alpha-tested
 // one, so scenes of at most kOnePassMeshlets meshlets, counted once per
@@ -280,8 +281,9 @@ size_t reset_bytes_for(const lh_ctx* c) {
 // 395 and 498 -> 562, and with alpha-tested ones 88,261 459 -> 564.
 constexpr uint64_t kOnePassMeshlets = 32768;
 uint32_t occlusion_px_of(const lh_ctx* c, uint32_t n_views) {
+    if (c->tuning.occlusion_px != LH_OCCLUSION_PX_DEFAULT) return c->tuning.occlusion_px;
     const uint64_t visibility_views = n_views > 4 ? n_views - 4 : 1;
-    return c->scene_meshlets * visibility_views <= kOnePassMeshlets ? 0u : c->tuning.occlusion_px;
+    return c->scene_meshlets * visibility_views <= kOnePassMeshlets ? 0u : LH_OCCLUSION_PX_DEFAULT;
 }
 
 FrameDev frame_dev(const lh_ctx* c, uint32_t n_views, uint32_t n_instances) {
@@ -534,7 +536,7 @@ lh_status lh_create(const lh_config* config, lh_ctx** out) {
     if (!c) return LH_ERR_OUT_OF_MEMORY;
     c->cfg = cfg;
     c->device = cfg.device;
-    c->tuning = lh_tuning{32u, 32u, 3.0f, LH_SCHEDULE_DEFAULT, 0u, 128u, {16u, 32u}, {128u, 64u}, 8u};
+    c->tuning = lh_tuning{32u, 32u, 3.0f, LH_SCHEDULE_DEFAULT, 0u, LH_OCCLUSION_PX_DEFAULT, {16u, 32u}, {128u, 64u}, 8u};
     cudaError_t e = cudaSetDevice(c->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
     c->max_views = 5 + cfg.max_probes;
