@@ -256,7 +256,8 @@ typedef struct lh_tuning {
                                  reference; results identical).  0: one pass, no occlusion test.  The
                                  default, LH_OCCLUSION_PX_DEFAULT, draws scenes of at most 32,768 meshlets
                                  (times the visibility views) in one pass; any other value is taken as
-                                 it is */
+                                 it is (two passes pay in such a scene where large meshlets hide many
+                                 of some tens of pixels) */
     uint32_t chunk_rows[2];   /* pixel rows of a big-triangle chunk (one warp) in the visibility / shadow
                                  pass: 4, 8, 16 or 32 */
     uint32_t chunk_cols[2];   /* its columns: 32, 64, 128 or 256 */

@@ -270,15 +270,20 @@ size_t reset_bytes_for(const lh_ctx* c) {
 
 // The occluder threshold of a frame of n_views views (4 of them cascades): the
 // tuning's, or what suits the scene where it is the default.
-// The two-pass raster's four launches cost 13 to 30 us a frame; rasterising
-// what they would have skipped costs about 1 ns a meshlet, 5 an alpha-tested
-// one, so scenes of at most kOnePassMeshlets meshlets, counted once per
-// visibility view, take one pass.  Measured by launches: 3,840 meshlets at 640 x
-// 360 105 -> 91 us, 15,360 at 1280 x 720 116 -> 102, 35,145 (two thirds of the
-// visible ones hidden) 189 -> 161, 44,496 258 -> 232, 145,845 290 -> 262; half
-// of them alpha-tested: 1,200 101 -> 89 us, 15,360 189 -> 174, 25,920 183 ->
-// 168, 27,993 283 -> 267.  The other way round 595,594 at 1920 x 1080 336 ->
-// 395 and 498 -> 562, and with alpha-tested ones 88,261 459 -> 564.
+// The two-pass raster's four launches cost 13 to 37 us a frame; rasterising
+// what they would have skipped costs about 1 ns a meshlet whose triangles hold no
+// pixel centre, 5 an alpha-tested one, so by default scenes of at most
+// kOnePassMeshlets meshlets, counted once per visibility view, take one pass.
+// Measured, two passes -> one: 3,840 meshlets at 640 x 360 105 -> 91 us, 15,360 at
+// 1280 x 720 116 -> 102, at 3840 x 2160 216 -> 194, 8,112 to 17,159 there 309-460
+// -> 277-434; half of them alpha-tested: 1,200 101 -> 89, 15,360 189 -> 174,
+// 25,920 183 -> 168, 27,993 283 -> 267.  Opaque scenes gain beyond the line too
+// (35,145 189 -> 161, 145,845 290 -> 262; 595,594 lose, 336 -> 395), alpha-tested
+// ones do not (88,261 459 -> 564): one line serves both.
+// The count does not see what is hidden: behind a wall of large meshlets, meshlets
+// of 40 x 40 pixels lose far more than the launches cost (3,072 at 1280 x 720 169
+// -> 204, 17,408 171 -> 461, 20,736 at 1920 x 1080 262 -> 589).  Scenes like that
+// want a threshold of their own, which is taken as it is.
 constexpr uint64_t kOnePassMeshlets = 32768;
 uint32_t occlusion_px_of(const lh_ctx* c, uint32_t n_views) {
     if (c->tuning.occlusion_px != LH_OCCLUSION_PX_DEFAULT) return c->tuning.occlusion_px;
