@@ -51,7 +51,7 @@ struct lh_ctx {
     uint8_t* d_sectors = nullptr;
     MeshletReference* d_refs = nullptr;
     RasterDraw* d_rdraws = nullptr;  // the raster's per-slot draw records
-    uint32_t* d_lists = nullptr;     // the views' raster lists (4 * max_draws words each)
+    uint32_t* d_lists = nullptr;     // the views' raster lists (ViewList), the cascades' first
     uint32_t* d_hiz = nullptr;       // hierarchical depth of the visibility views (pool)
     size_t hiz_words = 0;
     uint8_t* d_draws = nullptr;
@@ -245,7 +245,7 @@ void build_views(lh_ctx* c, uint32_t n_probes, const Uniforms* probe_uniforms) {
         vw.inst_status = reinterpret_cast<uint64_t*>(r + 4 * kClaimWords);
         vw.ml_status = reinterpret_cast<uint64_t*>(r + 4 * kClaimWords + 8 * (size_t)n_inst_tiles);
         vw.ml_tile_cap = ml_tiles;
-        vw.lists = c->d_lists + (size_t)v * 4 * cfg.max_draws;
+        vw.lists = c->d_lists + (cascade ? vw.cascade : 4 + (size_t)v * kViewLists) * cfg.max_draws;
         if (!cascade) {
             // the view's hierarchical depth from the pool while it lasts (a
             // view without one culls nothing)
@@ -559,7 +559,7 @@ lh_status lh_create(const lh_config* config, lh_ctx** out) {
     if (e == cudaSuccess) e = dalloc(c, &c->d_sectors, c->sector_bytes * c->max_views);
     if (e == cudaSuccess) e = dalloc(c, &c->d_refs, sizeof(MeshletReference) * 2 * (size_t)cfg.max_draws * c->max_views);
     if (e == cudaSuccess) e = dalloc(c, &c->d_rdraws, sizeof(RasterDraw) * 2 * (size_t)cfg.max_draws * c->max_views);
-    if (e == cudaSuccess) e = dalloc(c, &c->d_lists, sizeof(uint32_t) * 4 * (size_t)cfg.max_draws * c->max_views);
+    if (e == cudaSuccess) e = dalloc(c, &c->d_lists, sizeof(uint32_t) * (4 + kViewLists * (size_t)(1 + cfg.max_probes)) * cfg.max_draws);
     // hierarchical depth: the main view, and the probes' total pixels in 64 x
     // 64 regions with room for each probe's partial regions
     c->hiz_words = align_up(((W + kHizRegion - 1) / kHizRegion) * ((H + kHizRegion - 1) / kHizRegion) * 65, 64) +

@@ -172,7 +172,7 @@ __device__ __forceinline__ RasterDraw raster_draw_of(const FrameDev& f, const Vi
         if (occlusion && !alpha && (!(w > R) || radius_px > (float)f.occlusion_px * (w - R))) {
             r.bits |= kDrawOccluder;
             const uint32_t pos = count_up(&vw->claim[kClaimOccluders]);
-            if (pos < f.max_draws) vw->lists[pos] = slot;
+            if (pos < f.max_draws) vw->lists[(size_t)kSlotsOccluders * f.max_draws + pos] = slot;
         }
     } else {
         // an orthographic cascade: the matrix's y row scales to ndc
@@ -182,7 +182,7 @@ __device__ __forceinline__ RasterDraw raster_draw_of(const FrameDev& f, const Vi
     // (the occlusion raster lists its general meshlets after the depth test)
     if ((r.bits & kDrawGeneral) && !alpha && !occlusion) {
         const uint32_t pos = count_up(&vw->claim[kClaimGeneral]);
-        if (pos < f.max_draws) vw->lists[(size_t)3 * f.max_draws + pos] = slot;
+        if (pos < f.max_draws) vw->lists[(size_t)kSlotsGeneral * f.max_draws + pos] = slot;
     }
     return r;
 }

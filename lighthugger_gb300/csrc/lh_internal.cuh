@@ -60,12 +60,13 @@ constexpr uint32_t kDrawGeneral = 1u << 29;
 constexpr float kSmallRadiusPx = LH_SMALL_RADIUS_PX;
 constexpr uint32_t kNoCentreTestPixels = 512u * 512u;  // views up to this size test it (sphere_box.cuh)
 
-// Per-view lists of the two-pass occlusion raster of visibility views
-// (ViewDev::lists, 4 * max_draws words): draw slots of the occluders, then
-// of the opaque and the alpha-clip meshlets that survive the hierarchical
-// depth test, then of the opaque kDrawGeneral ones (survivors; in a view
-// without the occlusion raster, all of them).  Their counts are
+// A view's lists of draw slots (ViewDev::lists, max_draws words each; a cascade
+// has the first alone): the opaque kDrawGeneral meshlets (survivors; in a view
+// without the occlusion raster, all of them), then, of the two-pass occlusion
+// raster of visibility views, the occluders, and the opaque and the alpha-clip
+// meshlets that survive the hierarchical depth test.  Their counts are
 // ViewDev::claim[kClaimOccluders ...].
+enum ViewList : uint32_t { kSlotsGeneral = 0, kSlotsOccluders = 1, kSlotsOpaque = 2, kSlotsAlpha = 3, kViewLists = 4 };
 enum RasterList : uint32_t { kListAll = 0, kListOccluders = 1, kListSurvivors = 2 };
 enum ClaimWord : uint32_t {
     kClaimInstTiles = 0,
@@ -99,7 +100,7 @@ struct ViewDev {
     uint32_t* claim;            // per-frame zeroed kClaimWords: tile claims, occlusion list counts
     uint32_t section_base;      // firstInstance offset of this view's reference section
     uint32_t ml_tile_cap;       // capacity of ml_status
-    uint32_t* lists;            // draw-slot lists of the raster passes (RasterList; 4 * max_draws)
+    uint32_t* lists;            // draw-slot lists of the raster passes (ViewList)
     uint32_t* hiz;              // visibility views with occlusion culling: hierarchical depth, else null
     uint32_t hiz_rx, hiz_ry;    // 64 x 64-pixel regions of the view
 };

@@ -1177,7 +1177,8 @@ __device__ __forceinline__ uint32_t raster_list_count(const FrameDev& f, const V
 __device__ __forceinline__ const uint32_t* raster_list(const FrameDev& f, const ViewDev* vw, bool alpha, uint32_t list,
                                                        RasterLoop loop) {
     if (list == kListAll && (alpha || loop == kLoopSmall)) return nullptr;
-    const uint32_t k = list == kListOccluders ? 0u : alpha ? 2u : loop == kLoopGeneral ? 3u : 1u;
+    const uint32_t k = list == kListOccluders ? kSlotsOccluders
+                       : alpha ? kSlotsAlpha : loop == kLoopGeneral ? kSlotsGeneral : kSlotsOpaque;
     return vw->lists + (size_t)k * f.max_draws;
 }
 
@@ -2127,7 +2128,7 @@ __device__ void phase_occlusion_filter(const FrameDev& f, uint32_t view_begin, u
         // whole warps iterate together (the appends are warp collectives)
         for (uint64_t base = gtid - lane; base < n; base += gstride) {
             const uint64_t i = base + lane;
-            uint32_t cl = 0, slot = 0;  // the survivor list's number, 0: culled
+            uint32_t cl = kSlotsOccluders, slot = 0;  // the list it joins; none: an occluder, or culled
             if (i < n) {
                 const bool alpha = i >= nop;
                 slot = alpha ? md + (uint32_t)(i - nop) : (uint32_t)i;
@@ -2137,17 +2138,20 @@ __device__ void phase_occlusion_filter(const FrameDev& f, uint32_t view_begin, u
                 const float4 sp4 = __ldcg(reinterpret_cast<const float4*>(rd->sphere));
                 if (!(bits & (kDrawOccluder | kDrawNoCentre))) {
                     const float sp[4] = {sp4.x, sp4.y, sp4.z, sp4.w};
-                    if (!vw->hiz || !hiz_occluded(vw, pv, sp)) cl = alpha ? 2u : (bits & kDrawGeneral) ? 3u : 1u;
+                    if (!vw->hiz || !hiz_occluded(vw, pv, sp)) cl = alpha ? kSlotsAlpha : (bits & kDrawGeneral) ? kSlotsGeneral : kSlotsOpaque;
                 }
             }
 #pragma unroll
-            for (uint32_t k = 1; k <= 3; k++) {
+            for (uint32_t k = 0; k < kViewLists; k++) {
+                if (k == kSlotsOccluders) continue;
                 const uint32_t m = __ballot_sync(0xFFFFFFFFu, cl == k);
                 if (!m) continue;
                 const uint32_t leader = __ffs(m) - 1;
                 uint32_t first = 0;
                 if (lane == leader)
-                    first = atomicAdd(&vw->claim[k == 1 ? kClaimSurvivorsOpaque : k == 2 ? kClaimSurvivorsAlpha : kClaimGeneral],
+                    first = atomicAdd(&vw->claim[k == kSlotsOpaque  ? kClaimSurvivorsOpaque
+                                                 : k == kSlotsAlpha ? kClaimSurvivorsAlpha
+                                                                    : kClaimGeneral],
                                       __popc(m));
                 first = __shfl_sync(0xFFFFFFFFu, first, leader);
                 const uint32_t pos = first + __popc(m & ((1u << lane) - 1u));
