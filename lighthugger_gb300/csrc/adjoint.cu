@@ -396,16 +396,17 @@ __device__ __forceinline__ void pixel_backward(const FrameDev& f, const float4* 
 // The four texels of one bilinear sample (00, 10, 01, 11): summed over the
 // run of pixels along the warp that sample the same four, and added to the
 // texture's gradient image, channels [c0, c0 + NC).  Equal first texels of
-// one texture have equal others, so one look at the runs serves all four
-// (each by itself: 120 us of the kernel's 470 at 1920 x 1080, 74 so).  In a
-// texture one texel wide or high, taps on the same texel are merged.
+// one texture (`index`; others may share its image) have equal others, so one
+// look at the runs serves all four (each by itself: 120 us of the kernel's
+// 470 at 1920 x 1080, 74 so).  In a texture one texel wide or high, taps on the
+// same texel are merged.
 template <int NC>
-__device__ __forceinline__ void scatter_texels(HotCache& cache, float* dst, const lh_texture& t, const int32_t ij[4],
+__device__ __forceinline__ void scatter_texels(HotCache& cache, float* dst, const lh_texture& t, uint32_t index, const int32_t ij[4],
                                                float v[4][NC], int c0) {
     const int32_t W = dst ? (int32_t)t.width : 0;
     float* const first = dst ? dst + 4 * ((size_t)ij[2] * W + ij[0]) : nullptr;
     if (!__any_sync(kFull, first != nullptr)) return;
-    const Run r = run_of((unsigned long long)first);
+    const Run r = run_of((unsigned long long)first ^ ((unsigned long long)index << 48));  // (addresses have 48 bits)
     if (r.span > 1) {
         float s[4 * NC];
 #pragma unroll
@@ -533,8 +534,8 @@ __global__ void __launch_bounds__(32 * ROWS, LH_BWD_MIN_BLOCKS * 8 / ROWS)
             const uint32_t mi = o.ok && g.mr_index < f.n_textures ? g.mr_index : 0u;
             float* base = o.ok && g.base_index < f.n_textures ? reinterpret_cast<float*>(tex_targets[bi]) : nullptr;
             float* mr = o.ok && g.mr_index < f.n_textures ? reinterpret_cast<float*>(tex_targets[mi]) : nullptr;
-            scatter_texels<3>(cache, base, f.textures[bi], g.base_ij, g.base_texel, 0);
-            scatter_texels<2>(cache, mr, f.textures[mi], g.mr_ij, g.mr_texel, 1);  // roughness (g), metallic (b)
+            scatter_texels<3>(cache, base, f.textures[bi], bi, g.base_ij, g.base_texel, 0);
+            scatter_texels<2>(cache, mr, f.textures[mi], mi, g.mr_ij, g.mr_texel, 1);  // roughness (g), metallic (b)
         }
         // the geometry half of the reverse, then the vertex attributes: one
         // run per triangle
