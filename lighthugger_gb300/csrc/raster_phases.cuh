@@ -1082,7 +1082,8 @@ __device__ __forceinline__ SmallResult raster_meshlet_small(const FrameDev& f, c
                     const int32_t Px = s.kx0 * 256, Py = s.ky0 * 256;
                     int32_t e12 = (s.cy - s.by) * (Px - s.bx) - (s.cx - s.bx) * (Py - s.by);
                     int32_t e20 = (s.ay - s.cy) * (Px - s.cx) - (s.ax - s.cx) * (Py - s.cy);
-                    int32_t e01 = s.A - e12 - e20 + s.n01;
+                    // (unsigned: a sum on the way may wrap)
+                    int32_t e01 = (int32_t)((uint32_t)s.A - (uint32_t)e12 - (uint32_t)e20 + (uint32_t)s.n01);
                     e12 += s.n12;
                     e20 += s.n20;
                     const int32_t x12 = (s.cy - s.by) * 256, x20 = (s.ay - s.cy) * 256;
@@ -1727,13 +1728,11 @@ __device__ __noinline__ uint32_t raster_chunk_alpha(const FrameDev& f, const Big
     }
 }
 
-// One warp per chunk of a big triangle (rows x columns of f.chunk_shift,
-// at most 32 x 256 pixels): opaque chunks by runs of covered pixels
-// (raster_chunk_runs), alpha-tested ones pixel by pixel, skipped whole when
-// their rectangle lies outside one edge.
 // The opaque or alpha-tested pixels [x0, x1] x [y0, y1] (at most 32 x 256) of
-// the big triangle `b` (queue entry `entry`), by the whole warp; returns the
-// fragments this lane counts.
+// the big triangle `b` (queue entry `entry`), by the whole warp: opaque ones by
+// runs of covered pixels (raster_chunk_runs), alpha-tested ones pixel by pixel
+// unless the rectangle lies outside one edge.  Returns the fragments this lane
+// counts.
 template <int KIND>
 __device__ __forceinline__ uint32_t raster_chunk(const FrameDev& f, const BigTri& b, const BigTri* entry, const ChunkSteps& ks,
                                                  int32_t x0, int32_t x1, int32_t y0, int32_t y1, uint32_t lane, void* target,
