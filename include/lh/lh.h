@@ -247,8 +247,8 @@ typedef struct lh_tuning {
                                  chunk_cols pixels, one warp each) */
     float cull_blocks_per_sm; /* meshlet-cull blocks per SM (per-stage schedule); blocks per SM (persistent) */
     uint32_t schedule;        /* LH_SCHEDULE_* */
-    uint32_t raster_batch;    /* meshlets a raster warp claims per atomic, at most 8 (0: from 8 down to 1 as the
-                                 meshlets of the views run out) */
+    uint32_t raster_batch;    /* meshlets a raster warp claims per atomic (0: from 8 down to 1 as the meshlets
+                                 of the views run out; 9 to 64 are accepted and act as 8) */
     uint32_t occlusion_px;    /* two-pass occlusion raster of the visibility views: opaque meshlets whose
                                  bounding sphere projects to a radius above this many pixels are drawn
                                  first, the hierarchical depth of what they wrote is built, and every other
@@ -291,17 +291,17 @@ lh_status lh_get_stage_times(lh_ctx* ctx, float* ms, uint32_t n);
  * (passed to the kernel by value).  Output: a caller-owned prefix sector
  * {u64 counter; PrefixSumValue[capacity]} in device memory, identical to
  * lh_frame's main-view sector.  `d_flags` (optional, device) receives
- * LH_FLAG_* bits.  The kernel's scratch is a fixed array inside the library
- * of about 33 KB per GPU, so n_instances is limited to 1,048,576
- * (LH_ERR_CAPACITY beyond).  A call outside stream capture looks up that
- * array's address on the current device; a call during capture reuses the
- * address found by the last call outside capture (LH_ERR_UNSUPPORTED if there
- * was none), so the first call on a device should come before any stream
- * capture.  All calls share the array, so calls that overlap on the GPU
- * race -- serialise them.  Every block ORs the flags it raises into d_flags
- * itself (LH_FLAG_TIMEOUT, LH_FLAG_INSTANCE_OVERFLOW); with more visible
- * instances than `capacity` the counter holds the true count and entries
- * stop at `capacity`. */
+ * LH_FLAG_* bits.  The scratch of calls above 4,096 instances is a fixed array
+ * inside the library of about 8 KB per GPU, so n_instances is limited to
+ * 1,048,576 (LH_ERR_CAPACITY beyond).  A call outside stream capture looks up
+ * that array's address on the current device, whatever its size; a call during
+ * capture reuses the address found by the last call outside capture
+ * (LH_ERR_UNSUPPORTED if there was none), so the first call on a device should
+ * come before any stream capture.  Calls above 4,096 instances share the array, so
+ * those that overlap on the GPU race -- serialise them.  The kernel ORs the flags
+ * it raises into d_flags itself (LH_FLAG_INSTANCE_OVERFLOW, and above 4,096
+ * instances LH_FLAG_TIMEOUT); with more visible instances than `capacity` the
+ * counter holds the true count and entries stop at `capacity`. */
 lh_status lh_cull_instances_noalloc(const Instance* d_instances, uint32_t n_instances,
                                     const Uniforms* host_uniforms, uint8_t* d_sector, uint32_t capacity,
                                     uint32_t* d_flags, void* stream);

@@ -32,10 +32,13 @@ LH_FACING_HD bool faces_away(float nx, float ny, float nz, float vx, float vy, f
 
 // Whether a normal cone is seen from behind: dot(d', a') >= cutoff, where d' is
 // d normalised (`unit`: d as it is) and a' is a normalised `times` times, in IEEE
-// arithmetic.  Twelve divisions and roots lie behind that; their rounding, and
-// that of the approximate reciprocal roots here, moves the product by less
-// than 2^-20 of the sum of its terms' magnitudes, so they are only taken
-// nearer than 2^-18 to the cutoff, or for extreme lengths.
+// arithmetic.  Twelve divisions and roots lie behind that.  In units of 2^-24 of
+// the sum of the terms' magnitudes their rounding moves the product by at most
+// 13.5 (3.5 for each of three normalisations, 3 for the products and sums), that
+// of the approximate reciprocal roots here by 16 (4 for each of two, 3 for the
+// squared lengths, 2 for the scaling, 3 for the products and sums): less than
+// 2^-19 together, so the plain form decides nearer than 2^-18 to the cutoff, or
+// for extreme lengths.
 LH_FACING_HD bool cone_behind_ieee(const float* d, const float* a, float cutoff, bool unit, int times) {
     float x = a[0], y = a[1], z = a[2], u = d[0], v = d[1], w = d[2];
     for (int i = 0; i < times; i++) {

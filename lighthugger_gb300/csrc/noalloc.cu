@@ -19,7 +19,7 @@
 //    the address kept by the last call outside capture, so make the first
 //    call on a device before any stream capture (after a cudaDeviceReset,
 //    or under another context, make one call outside capture again);
-//  - every call shares the one array: calls whose work overlaps on the GPU
+//  - every call above 4,096 instances shares the one array: calls whose work overlaps on the GPU
 //    (different streams, or different host threads) race on it and give
 //    wrong results; serialise them;
 //  - each call clears the array on its own stream before the kernel runs
@@ -60,9 +60,9 @@ std::atomic<unsigned long long*> g_scratch_ptr[kMaxDevices];
 // stride reaches the memory system, and a record is read from shared memory
 // without bank conflicts (28 words a lane: the 8 lanes of a 16-byte access
 // phase start 4 banks apart).  700,001 instances inside a graph: 35 us by tiles
-// of 256, 33 by 512, 28 by 1,024 (4,097: 4.4, 4.9 and 5.3); a call by itself 52
-// with each thread's own loads and a look-back of one predecessor at a time,
-// 35 now.
+// of 256, 33 by 512, 28 by 1,024 (4,097: 4.4, 4.9 and 5.3); a call by itself 50 to
+// 52 with each thread's own loads and a look-back of one predecessor at a time, 35
+// to 37.5 now.
 __global__ void __launch_bounds__(kCullTile) k_cull_instances_noalloc(const Instance* instances, uint32_t n,
                                                                     const __grid_constant__ Uniforms u, uint8_t* sector,
                                                                     uint32_t capacity, uint32_t* flags_out,

@@ -12,9 +12,10 @@
 namespace lh {
 namespace {
 
-// The opaque class.  Four resident blocks per SM (64 registers): the 1080p
-// frame 0.616 ms at three, 0.606 at four, 0.624 at five; the 4K stress frame
-// 18.3 / 17.8 / 18.0; main + 32 probes 2.28 / 2.29 / 2.35.
+// The opaque class.  Four resident blocks per SM (64 registers), at three /
+// four / five: main + 32 probes 1744 / 1677 / 1720 us, the 4K stress frame 10.12 /
+// 9.78 / 10.01 ms; frames of few meshlets are a little better at three (1080p
+// before walls 469 / 477 / 493 us, 512 x 512 training step 418 / 430 / 456).
 template <int KIND>
 __global__ void __launch_bounds__(kRasterWarps * 32, LH_RASTER_MIN_BLOCKS)
     k_raster(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune, uint32_t list) {

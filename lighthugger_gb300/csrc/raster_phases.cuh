@@ -1372,11 +1372,12 @@ __device__ __forceinline__ void raster_setup(const FrameDev& f, uint32_t view_be
         // Work units: a meshlet, or a quarter of its triangles when the views
         // hold fewer meshlets than the grid has warps.  Every quarter
         // transforms the meshlet's vertices again: with quarters up to two
-        // meshlets per warp a 720p frame of 64 small spheres (8,100 meshlets
-        // a view, 4,864 warps) took 0.151 ms, with this line 0.117.
+        // meshlets per warp a 720p frame of 64 small spheres (7,600 meshlets
+        // a view, 4,864 warps) takes 134 us, with this line 100.
         const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);
         // Meshlets of the general path have more work in their triangles:
-        // quarters up to two per warp (foliage frame, 0.71 against 0.85 ms).
+        // quarters up to two per warp (1080p before walls 476.5 against 477.5
+        // us, the rest the same either way).
         k.split_shift = run < (loop == kLoopGeneral ? 2u * warps_total : warps_total) ? 2u : 0u;
         k.n_units = run << k.split_shift;
         k.batch = tune.batch;
@@ -1940,12 +1941,16 @@ __device__ __forceinline__ void raster_big_whole(const FrameDev& f, BigSmem& sm,
 // The chunk queue: the large triangles' chunks first, then the whole
 // triangles, which fill the launch's end.  A claim of a chunk is a chain of an
 // atomic, a three-step search and an entry's load behind the warp's own
-// reductions; most triangles are one or two chunks, and a claim each left the
-// launch 40 % idle: 1080p frame of 40,000 queued triangles, visibility passes
-// 84 + 75 -> 60 + 57 us, cascades 159 -> 104 us with claims of several, the
-// chunks of a claim merged along their row, set-up in 32 bits where it fits
-// and both edge values of a pixel converted in one register pair; whole
-// triangles by index took the 4K stress frame 16.3 -> 15.9 ms after that.
+// reductions; most triangles are one or two chunks, so claims take several, the
+// chunks of a claim are merged along their row, and small triangles go whole,
+// by their index.  Limit of a whole triangle in the visibility pass, 0 / 1 / 2 / 3
+// chunks: the 4K stress frame 10.23 / 10.06 / 9.78 / 9.62 ms, 1080p before walls
+// 490 / 490 / 477 / 477 us, another 305 / 296 / 290 / 293.  Most chunks a claim
+// takes, 8 / 16 / 32 / 64: stress 9.95 / 9.83 / 9.78 / 9.79 ms, the rest the same.
+// Share of what is left that a claim takes (LH_CHUNK_SHIFT 31 / 32 / 33): 32 probes
+// 1719 / 1677 / 1681 us, before walls 472 / 477 / 477; the same of whole triangles
+// (LH_WHOLE_SHIFT): 1080p 320 / 310 / 311, another 281 / 290 / 290, before walls
+// 485 / 477 / 492, training step 428 / 430 / 437.
 template <int KIND>
 __device__ void phase_raster_big(const FrameDev& f, BigSmem& sm) {
     __syncthreads();  // `sm` may still be in use by a previous phase of the block
