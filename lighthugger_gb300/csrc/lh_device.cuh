@@ -26,8 +26,9 @@ namespace lh {
 // completed and its writes are visible, so nothing is read or written
 // early, and then lets the next kernel of the stream begin launching.  In a
 // kernel launched without the attribute both instructions return at once.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 

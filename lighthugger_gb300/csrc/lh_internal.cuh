@@ -172,14 +172,13 @@ struct FrameDev {
     uint32_t scene_alpha;       // some mesh of the scene is alpha clip (else no alpha-class launch)
 };
 
-// Launch `kernel` with programmatic stream serialisation: its blocks may
-// become resident while the previous kernel of the stream drains, hiding the
-// launch gap between the frame's kernels (the kernel must begin with
-// pdl_enter()).  Build with LH_PDL=0 for plain launches.  A launch that is
-// captured into a graph is a plain one: a graph's kernels follow one another
-// closely without it, and replayed with programmatic edges the 1080p frame
-// took 0.510-0.536 ms against 0.470-0.496 (four scenes; as launches it takes
-// 0.472 with them, 0.500 without).
+// Launch `kernel` with programmatic stream serialisation: its launch is
+// prepared, and its blocks may become resident, while the previous kernel of the
+// stream drains, hiding the gap between the frame's kernels (the kernel must begin
+// with pdl_enter(), or pdl_wait() where the one after it should not begin early).
+// Build with LH_PDL=0 for plain launches: the 1080p frame of the benchmark back to
+// back 363 us against 332.  A launch that is captured into a graph is a plain one:
+// a graph's kernels follow one another closely without it (330 us).
 #ifndef LH_PDL
 #define LH_PDL 1
 #endif

@@ -12,6 +12,13 @@
 namespace lh {
 namespace {
 
+// These kernels begin with pdl_wait, not pdl_enter: the next kernel's blocks do
+// not become resident while they run.  Their blocks hold most of an SM's
+// registers and shared memory and leave at different times, so early blocks of the
+// next kernel came to stand unevenly, on SMs whose shared memory was still split for
+// this one: by launches the 1080p frame of the benchmark took 359 or 391 us behind
+// an L2 flush from one frame to the next, 346 so; back to back 345 -> 332, another
+// 327 -> 312, foliage 411 -> 397, 32 probes 1736 -> 1688, none longer.
 // The opaque class.  Four resident blocks per SM (64 registers), at three /
 // four / five: main + 32 probes 1744 / 1677 / 1720 us, the 4K stress frame 10.12 /
 // 9.78 / 10.01 ms; frames of few meshlets are a little better at three (1080p
@@ -20,7 +27,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kRasterWarps * 32, LH_RASTER_MIN_BLOCKS)
     k_raster(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune, uint32_t list) {
     __shared__ RasterSmemSmall sm;
-    pdl_enter();
+    pdl_wait();
     phase_raster<KIND>(f, view_begin, n_views, tune, sm, list);
 }
 
@@ -28,7 +35,7 @@ __global__ void __launch_bounds__(kRasterWarps * 32, LH_RASTER_MIN_BLOCKS)
 __global__ void __launch_bounds__(kRasterWarps * 32, 3)
     k_raster_occluders(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune) {
     __shared__ RasterSmem sm;
-    pdl_enter();
+    pdl_wait();
     phase_raster_general<0, false>(f, view_begin, n_views, tune, sm, nullptr, kListOccluders);
 }
 
@@ -37,26 +44,26 @@ template <int KIND>
 __global__ void __launch_bounds__(kRasterWarps * 32, 3)
     k_raster_alpha(const __grid_constant__ FrameDev f, uint32_t view_begin, uint32_t n_views, RasterTune tune, uint32_t list) {
     __shared__ RasterSmemAlpha sm;
-    pdl_enter();
+    pdl_wait();
     phase_raster_general<KIND, true>(f, view_begin, n_views, tune, sm, sm.alpha, list);
 }
 
 template <int KIND>
 __global__ void __launch_bounds__(256, LH_RASTER_BIG_MIN_BLOCKS) k_raster_big(const __grid_constant__ FrameDev f) {
     __shared__ BigSmem sm;
-    pdl_enter();
+    pdl_wait();
     phase_raster_big<KIND>(f, sm);
 }
 
 // Hierarchical depth of the visibility views after the occluder pass.
 __global__ void __launch_bounds__(256) k_hiz(FrameDev f, uint32_t view_begin, uint32_t n_views) {
-    pdl_enter();
+    pdl_wait();
     phase_hiz(f, view_begin, n_views);
 }
 
 // Depth test of the other visible meshlets' spheres; survivor lists.
 __global__ void __launch_bounds__(256) k_occlusion_filter(FrameDev f, uint32_t view_begin, uint32_t n_views) {
-    pdl_enter();
+    pdl_wait();
     phase_occlusion_filter(f, view_begin, n_views, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
                            (uint64_t)gridDim.x * blockDim.x);
 }
