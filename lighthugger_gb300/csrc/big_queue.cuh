@@ -24,7 +24,9 @@ constexpr uint32_t kBiasWhole = 32u;  // BigTri: taken whole by one warp, not by
 // Shadow raster at limits 0 / 1 / 2 / 3, us: 1080p frame of the benchmark 75.7 /
 // 75.8 / 81.9 / 84.0, before walls 210.9 / 186-188 / 192.5 / 211-213, 512 x 512
 // training step 172-174 / 155.6 / 161.8 / 176.1; visibility raster at 1 / 2
-// before walls: 163.5 / 149.2.
+// before walls: 163.5 / 149.2.  Whole frames at a shadow limit of 1 / 2: 327 / 333,
+// 503 / 520, 341 / 351 (training step), 32 probes 1682 / 1690 and, the one that
+// loses, 1943 / 1932.
 #ifndef LH_WHOLE_CHUNKS
 #define LH_WHOLE_CHUNKS 2
 #endif
